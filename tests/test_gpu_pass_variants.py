@@ -1,0 +1,59 @@
+"""Launch shapes that depend on the size of the work: every shape gives the same bits, and the
+smallest one agrees with the FP64 oracle engine."""
+import numpy as np
+import pytest
+
+import mdpd
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+RHO = 6.05
+
+
+def lattice(n, L, seed):
+    """n sites of a jittered cubic lattice and Maxwell velocities"""
+    rng = np.random.default_rng(seed)
+    m = int(np.ceil(n ** (1 / 3)))
+    s = rng.permutation(m ** 3)[:n]
+    x = (np.stack([s % m, s // m % m, s // m // m], 1) + 0.5 + rng.uniform(-0.3, 0.3, (n, 3))) * (L / m)
+    v = rng.normal(0, 1, (n, 3))
+    return x, v - v.mean(0)
+
+
+# the box sizes: a row block cut short (401 = 3 x 128 + 17), whole blocks, one row past a block
+@pytest.mark.parametrize("n", [401, 2048, 2049])
+@pytest.mark.parametrize("exact", [0, 1])
+def test_small_box_same_bits_in_any_mix_and_close_to_the_oracle(n, exact):
+    """alone the box takes the shapes of the smallest work; beside boxes of 20k, 100k and 700k
+    particles those of the larger ranges"""
+    L = (n / RHO) ** (1 / 3)
+    x, v = lattice(n, L, 5)
+    spec = mdpd.box_spec(n, L, x=x, v=v, seed=77, exact_rng=exact)
+    got = []
+    for other in (0, 20000, 100000, 700000):
+        sp = [spec]
+        if other:
+            sp.append(mdpd.box_spec(other, (other / RHO) ** (1 / 3), seed=5, init_seed=3, exact_rng=exact))
+        b = mdpd.Batch(sp)
+        b.setup()
+        b.step(5)
+        got.append(b.state(0))
+        b.step(7)
+        got[-1] += b.state(0)
+        b.close()
+    for g in got[1:]:
+        for a, c in zip(got[0], g):
+            assert np.array_equal(a, c)
+    # 5 steps, each adding to v at most dt times the force bar (1e-5 of the RMS force, ~60) and, with
+    # the FP32 gaussian, its error (3e-6) in ~25 random pair forces of sigma w_c / sqrt(dt) ~ 10 each;
+    # half as much again for growth
+    sim = oracle.Sim(x, v, (0, 0, 0), (L, L, L), seed=77)
+    sim.setup()
+    sim.run(5)
+    xo, vo = sim.state()[:2]
+    sim.close()
+    bar = 1.5 * 5 * 0.01 * (1e-5 * 60 + 25 * 10 * 3e-6)
+    assert np.abs(got[0][1] - vo).max() < bar
+    dx = got[0][0] - xo
+    assert np.abs(dx - L * np.round(dx / L)).max() < 5 * 0.01 * bar

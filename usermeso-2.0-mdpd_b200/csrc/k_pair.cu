@@ -11,8 +11,8 @@
 //   shifted in the positive direction).  The mirrored pair, seen from the other end, has the
 //   opposite shift, so every pair is owned by exactly one row.  It also writes (x, y, z, rho) of
 //   the particle and its ghost images for the force pass's gathers.
-// k_force_pairs: the 32 compact rows of a warp are concatenated and split into 32 equal
-//   contiguous shares, one per lane (a prefix scan of the row lengths and one binary search), so
+// k_force_pairs: the compact rows of a warp (32 of them; 4, 8 or 16 where that fills the chip
+//   better, force_rows) are concatenated and split into 32 equal contiguous shares, one per lane (a prefix scan of the row lengths and one binary search), so
 //   every lane evaluates the same number of pairs whatever the row lengths.  The concatenated
 //   rows are first staged in shared memory by coalesced loads (consecutive lanes, consecutive
 //   entries), so the pair loop's entry reads (each lane in a different row) do not touch 32
@@ -20,7 +20,7 @@
 //   two float4 gathers, loaded for the next pair while the current one is evaluated.  The mDPD pair force (pair_mdpd_meso.cu:139-225)
 //   is summed for the row in 64-bit fixed point (2^-32 units) in registers and flushed when the
 //   lane's share moves to the next row; -F goes to j's source particle in the same fixed point,
-//   through shared memory when the source is one of the block's 128 rows and global 64-bit
+//   through shared memory when the source is one of the block's rows and global 64-bit
 //   atomics otherwise.  Integer addition is associative, so no sum depends on the order of the
 //   atomics: results are bitwise reproducible and the pairwise forces cancel exactly (total
 //   momentum).  Every pair term is checked against the box's fix_pair_max, which keeps each
@@ -168,23 +168,23 @@ __device__ __forceinline__ unsigned long long join64(unsigned lo, unsigned hi)
     return ((unsigned long long)hi << 32) | lo;
 }
 
-// compact entries a warp stages in shared memory: its 32 rows hold ~400 at rho 6.05 (12.6 owned
-// force-range pairs each); a warp with more reads them from the table
-constexpr int kWarpEntries = 640;
+// compact entries a warp stages in shared memory per row: rows hold 12.6 owned force-range pairs
+// at rho 6.05; a warp with more than RW times this reads them from the table
+constexpr int kRowEntries = 20;
 
-// shared memory of the global-index force pass
-struct RowsSmem {
+// shared memory of the force pass, RW rows per warp
+template <int RW> struct RowsSmem {
     PairCoeff coeff[kMaxTypes * kMaxTypes];
-    float4 pi[128], vi[128];
-    float rho[128];
+    float4 pi[4 * RW], vi[4 * RW];
+    float rho[4 * RW];
     int pre[4][33];
-    unsigned lo[3][128], hi[3][128];
+    unsigned lo[3][4 * RW], hi[3][4 * RW];
     double red[4][7];
-    int ent[4][kWarpEntries];  // each warp's concatenated compact rows (when they fit)
+    int ent[4][RW * kRowEntries];  // each warp's concatenated compact rows (when they fit)
 };
 
-// the warp's rows [wb, wb + 32) as one list of T entries split into 32 equal shares; P: prefix
-// of the row lengths (P[r] entries before row r, P[32] = T)
+// the warp's rows as one list of T entries split into 32 equal shares; P: prefix of the row
+// lengths (P[r] entries before row r, P[32] = T; len is 0 in lanes that hold no row)
 __device__ __forceinline__ void warp_prefix(int len, int lane, int *P)
 {
     int pre = len;
@@ -196,12 +196,12 @@ __device__ __forceinline__ void warp_prefix(int len, int lane, int *P)
     if (lane == 0) P[0] = 0;
 }
 
-// the row holding entry m of the concatenated rows: the last r with P[r] <= m
-__device__ __forceinline__ int row_of(const int *P, int m)
+// the row (of RW) holding entry m of the concatenated rows: the last r with P[r] <= m
+template <int RW> __device__ __forceinline__ int row_of(const int *P, int m)
 {
     int r = 0;
 #pragma unroll
-    for (int st = 16; st > 0; st >>= 1)
+    for (int st = RW / 2; st > 0; st >>= 1)
         if (P[r + st] <= m) r += st;
     return r;
 }
@@ -222,23 +222,26 @@ __device__ __forceinline__ void ev_to_partial(const BoxDesc &B, const Unit &U, c
     }
 }
 
-template <bool EXACT, bool EV, bool UNI>
-__device__ __forceinline__ void force_pairs(const BoxDesc &B, const Unit &U, RowsSmem &S, int stage_cap)
+// rows [U.begin, U.end) of one block: 4 RW of them at most
+template <bool EXACT, bool EV, bool UNI, int RW>
+__device__ __forceinline__ void force_pairs(const BoxDesc &B, const Unit &U, RowsSmem<RW> &S, int stage_cap)
 {
-    const int t = threadIdx.x, lane = t & 31, w = t >> 5, wb = t & ~31;
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5, wb = w * RW;
     for (int q = t; q < (UNI ? 1 : B.ntype * B.ntype); q += blockDim.x) S.coeff[q] = B.coeff[q];
-    const int i = U.begin + t;
-    const bool live = i < U.end;
+    // lanes below RW hold the warp's rows
+    const int row = wb + lane, i = U.begin + row;
+    const bool live = lane < RW && i < U.end;
     int len = 0;
     if (live) {
         prefetch_l2(B.table2 + (size_t)i * B.n_col2);  // the row's first 32 entries: one line
-        S.pi[t] = B.pos[i];
-        S.vi[t] = B.vel[i];
-        S.rho[t] = B.rho[i];
+        S.pi[row] = B.pos[i];
+        S.vi[row] = B.vel[i];
+        S.rho[row] = B.rho[i];
         len = MDPD_IDX(B.count2[i], B.n_col2 + 1);
     }
     warp_prefix(len, lane, S.pre[w]);
-    for (int c = 0; c < 3; ++c) S.lo[c][t] = S.hi[c][t] = 0u;
+    if (lane < RW)
+        for (int c = 0; c < 3; ++c) S.lo[c][row] = S.hi[c][row] = 0u;
     __syncthreads();
     const int *P = S.pre[w];
     const int T = P[32];
@@ -255,13 +258,13 @@ __device__ __forceinline__ void force_pairs(const BoxDesc &B, const Unit &U, Row
     int *const ent = S.ent[w];
     if (staged) {
         for (int m = lane; m < T; m += 32) {
-            const int r = row_of(P, m);
+            const int r = row_of<RW>(P, m);
             ent[m] = __ldcs(B.table2 + (size_t)(i0 + r) * ncol2 + (m - P[r]));
         }
         __syncwarp();
     }
     if (m0 < m1) {
-        int r = row_of(P, m0);
+        int r = row_of<RW>(P, m0);
         int rbeg = P[r], rend = P[r + 1];
         float4 pi = S.pi[wb + r], vi = S.vi[wb + r];
         float rho_i = S.rho[wb + r];
@@ -317,7 +320,7 @@ __device__ __forceinline__ void force_pairs(const BoxDesc &B, const Unit &U, Row
             const long long qx = to_fix(px), qy = to_fix(py), qz = to_fix(pz);
             ax += qx, ay += qy, az += qz;
             const int d = src - U.begin;
-            if ((unsigned)d < 128u) {  // one of this block's rows (src < nlocal, so d < U.end - U.begin)
+            if ((unsigned)d < (unsigned)(4 * RW)) {  // one of this block's rows (src < nlocal)
                 sadd64(&S.lo[0][d], &S.hi[0][d], -qx);
                 sadd64(&S.lo[1][d], &S.hi[1][d], -qy);
                 sadd64(&S.lo[2][d], &S.hi[2][d], -qz);
@@ -334,24 +337,27 @@ __device__ __forceinline__ void force_pairs(const BoxDesc &B, const Unit &U, Row
     if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&B.st->status, kErrNonFinite);
     __syncthreads();
     if (live) {
-        atomicAdd(fax + i, join64(S.lo[0][t], S.hi[0][t]));
-        atomicAdd(fay + i, join64(S.lo[1][t], S.hi[1][t]));
-        atomicAdd(faz + i, join64(S.lo[2][t], S.hi[2][t]));
+        atomicAdd(fax + i, join64(S.lo[0][row], S.hi[0][row]));
+        atomicAdd(fay + i, join64(S.lo[1][row], S.hi[1][row]));
+        atomicAdd(faz + i, join64(S.lo[2][row], S.hi[2][row]));
     }
     if (EV) ev_to_partial<EV>(B, U, ev, S.red);
 }
 
 // 7 blocks per SM (up to 72 registers, no spill) measured fastest against 6 and 8
-template <bool EXACT, bool EV, bool UNI>
+template <bool EXACT, bool EV, bool UNI, int RW>
 __global__ void __launch_bounds__(128, 7) k_force_pairs(const BoxDesc *__restrict__ boxes,
-                                                        const Unit *__restrict__ units, int nunits,
-                                                        int stage_cap)
+                                                        const Unit *__restrict__ units, int nunits, int staged)
 {
-    __shared__ RowsSmem S;
-    const int u = blockIdx.x;
+    static_assert(!EV || RW == 32, "the energy and virial partials are per unit");
+    __shared__ RowsSmem<RW> S;
+    constexpr int kParts = 32 / RW;  // blocks per unit
+    const int u = blockIdx.x / kParts;
     if (u >= nunits) return;
-    const Unit U = units[u];
-    force_pairs<EXACT, EV, UNI>(boxes[U.box], U, S, min(stage_cap, kWarpEntries));
+    Unit U = units[u];
+    U.begin += (blockIdx.x % kParts) * (4 * RW);
+    if (U.begin >= U.end) return;
+    force_pairs<EXACT, EV, UNI, RW>(boxes[U.box], U, S, staged ? RW * kRowEntries : 0);
 }
 
 __global__ void __launch_bounds__(kUnit) k_finalize(const BoxDesc *__restrict__ boxes,
@@ -406,25 +412,60 @@ void launch_density_half(cudaStream_t s, BoxDesc *boxes, const BatchUnits &u, co
     }
 }
 
-template <bool EXACT, bool EV, bool UNI>
-static void force_half(cudaStream_t s, BoxDesc *boxes, const BatchUnits &u, int stage_cap)
+template <bool EXACT, bool EV, bool UNI, int RW>
+static void force_half(cudaStream_t s, BoxDesc *boxes, const BatchUnits &u, int staged)
 {
-    k_force_pairs<EXACT, EV, UNI><<<u.local.n, 128, 0, s>>>(boxes, u.local.d, u.local.n, stage_cap);
+    k_force_pairs<EXACT, EV, UNI, RW><<<u.local.n * (32 / RW), 128, 0, s>>>(boxes, u.local.d, u.local.n, staged);
+}
+
+// Rows per warp of the force pass.  A lane walks its share of the warp's pairs one after another
+// (12.6 pairs at 32 rows and rho 6.05, ~2 us each with the loads they wait for), so while the
+// chip is not full fewer rows per warp shorten the pass: the fewest with which every block is
+// still resident at once (7 per SM).  Past that, up to a few resident waves, 16 rows lose less in
+// the last wave; beyond, 32 rows are best: shares are evener, rows change less often and more
+// partners are rows of the block, so fewer sums go through global atomics.  Force pass with
+// finalize, us at 32 / 16 / 8 / 4 rows:
+//       2,000 particles   32 /  21 /  15 /  13        8,000   32 /  21 /  17 /  14
+//      20,000             32 /  22 /  17 /  20       42,000   33 /  25 /  26 /  27
+//     200,000             72 /  64 /  70 /  87      500,000  137 / 134 / 160 / 207
+//   1,000,000            252 / 255 / 320 / 421    4,000,000  888 / 955 / 1242 / 1645
+// (a 109,000-particle slab, 0.8 waves at 32 rows: 1 us a step slower at 16).
+// The sums are fixed point, so every shape gives the same bits.
+static int force_rows(int nunits, int sms)
+{
+    const int resident = 7 * sms;
+    if (nunits * 8LL <= resident) return 4;
+    if (nunits * 4LL <= resident) return 8;
+    if (nunits * 2LL <= resident) return 16;
+    return nunits > resident && nunits <= 4LL * resident ? 16 : 32;
+}
+
+template <bool EXACT, bool UNI>
+static void force_half_rows(cudaStream_t s, BoxDesc *boxes, const BatchUnits &u, int rows, int staged)
+{
+    switch (rows) {
+    case 4: force_half<EXACT, false, UNI, 4>(s, boxes, u, staged); break;
+    case 8: force_half<EXACT, false, UNI, 8>(s, boxes, u, staged); break;
+    case 16: force_half<EXACT, false, UNI, 16>(s, boxes, u, staged); break;
+    default: force_half<EXACT, false, UNI, 32>(s, boxes, u, staged); break;
+    }
 }
 
 void launch_force_half(cudaStream_t s, BoxDesc *boxes, const BatchUnits &u, const StepConfig &c, int ev, int kick)
 {
     const int g = u.local.n;
     if (g <= 0) return;
-    const int cap = c.stage_rows ? kWarpEntries : 0;
-    if (c.exact_rng) {
-        if (ev) force_half<true, true, false>(s, boxes, u, cap);
-        else if (c.uniform_types) force_half<true, false, true>(s, boxes, u, cap);
-        else force_half<true, false, false>(s, boxes, u, cap);
+    const int staged = c.stage_rows;
+    const int rows = force_rows(u.local.n, c.sms);
+    if (ev) {
+        if (c.exact_rng) force_half<true, true, false, 32>(s, boxes, u, staged);
+        else force_half<false, true, false, 32>(s, boxes, u, staged);
+    } else if (c.exact_rng) {
+        if (c.uniform_types) force_half_rows<true, true>(s, boxes, u, rows, staged);
+        else force_half_rows<true, false>(s, boxes, u, rows, staged);
     } else {
-        if (ev) force_half<false, true, false>(s, boxes, u, cap);
-        else if (c.uniform_types) force_half<false, false, true>(s, boxes, u, cap);
-        else force_half<false, false, false>(s, boxes, u, cap);
+        if (c.uniform_types) force_half_rows<false, true>(s, boxes, u, rows, staged);
+        else force_half_rows<false, false>(s, boxes, u, rows, staged);
     }
     k_finalize<<<g, kUnit, 0, s>>>(boxes, u.local.d, g, kick);
 }
