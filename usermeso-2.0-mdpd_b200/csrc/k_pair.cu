@@ -456,7 +456,7 @@ void launch_force_half(cudaStream_t s, BoxDesc *boxes, const BatchUnits &u, cons
     const int g = u.local.n;
     if (g <= 0) return;
     const int staged = c.stage_rows;
-    const int rows = force_rows(u.local.n, c.sms);
+    const int rows = c.full_chip ? 32 : force_rows(u.local.n, c.sms);
     if (ev) {
         if (c.exact_rng) force_half<true, true, false, 32>(s, boxes, u, staged);
         else force_half<false, true, false, 32>(s, boxes, u, staged);

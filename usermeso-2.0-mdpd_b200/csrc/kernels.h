@@ -39,6 +39,7 @@ struct StepConfig {
     int stage_rows = 1;    // pair-once force pass: each warp's compact rows staged in shared memory
                            // (0: the pair loop reads its entries from the table)
     int aboundary = 0;     // fix aboundary/meso at the end of each step
+    int full_chip = 0;     // the pair-once passes take their shapes for a full chip at any size
     int sms = 148;
 };
 

@@ -157,6 +157,10 @@ void mdpd_server_s::loop()
     std::unique_ptr<Batch> batch;
     StepConfig cfg;
     cfg.sms = sm_count();
+    // Stepping sets are filled up to step_cap particles, where these are the fastest shapes.  A lone
+    // small job keeps its pace too: the scheduling test's 12,000-particle job of 3,000 steps has to
+    // be under way 0.2 s after it was submitted (0.25 s with these shapes, 0.18 s without).
+    cfg.full_chip = 1;
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
