@@ -57,3 +57,23 @@ def test_small_box_same_bits_in_any_mix_and_close_to_the_oracle(n, exact):
     assert np.abs(got[0][1] - vo).max() < bar
     dx = got[0][0] - xo
     assert np.abs(dx - L * np.round(dx / L)).max() < 5 * 0.01 * bar
+
+
+def test_ghost_overflow_is_reported_and_the_library_stays_usable():
+    """every particle within the ghost cutoff of a face: more images than the capacity estimated
+    for a uniform box"""
+    L = 40.0
+    n = int(RHO * 1.2 * L * L)
+    rng = np.random.default_rng(2)
+    x = rng.uniform(0, 1, (n, 3)) * (1.2, L, L)
+    b = mdpd.Batch([mdpd.box_spec(n, L, x=x, v=np.zeros((n, 3)))])
+    with pytest.raises(mdpd.MdpdError) as e:
+        b.setup()
+    assert e.value.code == mdpd.ERR_OVERFLOW and "ghost" in str(e.value)
+    b.close()
+    m = 2000
+    b = mdpd.Batch([mdpd.box_spec(m, (m / RHO) ** (1 / 3))])
+    b.setup()
+    b.step(3)
+    assert b.thermo(0).status == 0
+    b.close()

@@ -223,14 +223,14 @@ void Box::layout(const Spec &s, int na)
     B.cls_of = alloc<int>(n);
     B.sub_of = alloc<int>(n);
     B.perm = alloc<int>(n);
-    B.bin_of = alloc<int>(na);
+    B.bin_of = alloc<int>(n);
     B.bin_count = alloc<int>(nbin + 1);
     B.bin_start = alloc<int>(nbin + 1);
     B.bin_cursor = alloc<int>(nbin + 1);
     B.bin_order = alloc<int>(na);
     B.bpos = alloc<float4>(na);
-    const int nchunk = std::max({2 * nbin, n + 1, nbin}) / kScanChunk + 2;
-    B.scan_part = alloc<int>(nchunk);
+    B.scan_part = alloc<int>(2 * (size_t)nbin / kScanChunk + 1);
+    B.scan_part2 = alloc<int>((size_t)n / kScanChunk + 1);
     B.partial = alloc<double>((size_t)((n + kUnit - 1) / kUnit) * kPartialStride);
     d_state = alloc<BoxState>(1);
     B.st = d_state;
@@ -615,19 +615,21 @@ Batch::~Batch()
 static BatchUnits make_units(const std::vector<Box *> &boxes, const std::vector<int> &which, int nbox,
                              std::vector<Unit *> &allocs, cudaStream_t s)
 {
-    std::vector<Unit> loc, all, cls, bins, scls, sgh, sbin;
+    std::vector<Unit> loc, cls, bins, scls, sgh, sbin;
+    int longest_cls = 0, longest_ghost = 0;
     for (int b : which) {
         const BoxDesc &B = boxes[b]->desc;
         auto chunk = [&](std::vector<Unit> &v, int n, int step) {
             for (int s = 0; s < n; s += step) v.push_back({b, s, std::min(n, s + step)});
         };
         chunk(loc, B.nlocal, kUnit);
-        chunk(all, B.nlocal + B.ghost_cap, kUnit);
         chunk(cls, 2 * B.nbin, 256);
         chunk(bins, B.nbin, 256);
         chunk(scls, 2 * B.nbin, kScanChunk);
         chunk(sgh, B.nlocal + 1, kScanChunk);
         chunk(sbin, B.nbin, kScanChunk);
+        longest_cls = std::max(longest_cls, (2 * B.nbin - 1) / kScanChunk + 1);
+        longest_ghost = std::max({longest_ghost, B.nlocal / kScanChunk + 1, (B.nbin - 1) / kScanChunk + 1});
     }
     auto up = [&](const std::vector<Unit> &v) {
         Unit *d = batch_alloc<Unit>(v.size(), s);
@@ -638,12 +640,13 @@ static BatchUnits make_units(const std::vector<Box *> &boxes, const std::vector<
     };
     BatchUnits u;
     u.local = up(loc);
-    u.all = up(all);
     u.cls = up(cls);
     u.bins = up(bins);
     u.scan_cls = up(scls);
     u.scan_ghost = up(sgh);
     u.scan_bin = up(sbin);
+    u.longest_cls = longest_cls;
+    u.longest_ghost = longest_ghost;
     u.nbox = nbox;  // box-indexed kernels (scan tops, build counters) see every box of the batch
     check_cuda(cudaStreamSynchronize(s), "units");  // the host vectors above are the copies' sources
     return u;

@@ -7,12 +7,12 @@
 //            (sub key, original index).  Equals the reference's stable LSD radix sort of the
 //            full key (sort_meso.h:364-443), i.e. the same permutation.
 //   permute  gather every per-particle array into the other buffer, pack FP32 state,
-//            count ghost images of border particles, bin the locals
-//   ghosts   periodic images x + s*prd of every particle within cutghost of a face
-//            (MesoComm::borders, comm_meso.cu:42-193), binned with gpu_assign_bin_id's rule
-//            (neighbor_meso.cu:390-425)
+//            count ghost images of border particles, and the bins of locals and images
 //   bins     locals+ghosts by bin, index order inside a bin: a local's place follows from its
-//            reorder-class run; ghost images take atomic slots and bins holding them are sorted
+//            reorder-class run; ghost images, periodic images x + s*prd of every particle within
+//            cutghost of a face (MesoComm::borders, comm_meso.cu:42-193) binned with
+//            gpu_assign_bin_id's rule (neighbor_meso.cu:390-425), take atomic slots and bins
+//            holding them are sorted
 //   list     warp per bin: 27-bin stencil candidates filtered against the box of up to 32
 //            centres, then tested against each centre; every hit is written from the test
 //            ballot (atomic-free) straight into the locally transposed table, reduced rows on
@@ -83,39 +83,57 @@ __global__ void __launch_bounds__(kUnit) k_rb_key(const BoxDesc *__restrict__ bo
 }
 
 // ---------------------------------------------------------------------------
-// scans: per-box exclusive scans of a count array, three kernels without inter-block waits
+// scans: per-box exclusive scans of a count array in chunks of kScanChunk, without inter-block
+// waits.  A block finds what comes before its chunk by itself: by adding up the counts (short
+// scans: one kernel) or the chunk sums that a reduce kernel left (long ones: two kernels).
 // ---------------------------------------------------------------------------
-template <int SEL> __device__ __forceinline__ int *scan_in(const BoxDesc &B)
+// image counts of the locals: in cls_of, free once the class scatter has read it
+template <int SEL> __device__ __forceinline__ const int *scan_in(const BoxDesc &B)
 {
-    return SEL == kSelCls ? B.cls_count : SEL == kSelGhost ? B.gfirst : B.bin_count;
+    return SEL == kSelCls ? B.cls_count : SEL == kSelGhost ? B.cls_of : B.bin_count;
 }
+// elements in the array (the ghost scan has one output more)
 template <int SEL> __device__ __forceinline__ int scan_len(const BoxDesc &B)
 {
-    return SEL == kSelCls ? 2 * B.nbin : SEL == kSelGhost ? B.nlocal + 1 : B.nbin;
+    return SEL == kSelCls ? 2 * B.nbin : SEL == kSelGhost ? B.nlocal : B.nbin;
+}
+// first chunk with anything to scan: only border particles (from n_bulk on) have images
+template <int SEL> __device__ __forceinline__ int scan_first(const BoxDesc &B)
+{
+    return SEL == kSelGhost ? B.st->n_bulk / kScanChunk : 0;
+}
+template <int SEL> __device__ __forceinline__ int *scan_part(const BoxDesc &B)
+{
+    return SEL == kSelGhost ? B.scan_part2 : B.scan_part;
 }
 
-template <int SEL>
-__global__ void __launch_bounds__(256) k_scan_reduce(const BoxDesc *__restrict__ boxes,
-                                                     const Unit *__restrict__ units, int nunits)
+// sum over the block of 256 threads, in every thread
+__device__ __forceinline__ int block_sum_256(int a, int *s_w)
 {
-    __shared__ int s_w[8];
-    for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
-        const Unit U = units[u];
-        const BoxDesc &B = boxes[U.box];
-        if (!rebuilding(B)) continue;
-        const int *in = scan_in<SEL>(B);
-        int a = 0;
-        for (int k = U.begin + threadIdx.x; k < U.end; k += 256) a += in[k];
-        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-        if ((threadIdx.x & 31) == 0) s_w[threadIdx.x / 32] = a;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int t = 0;
-            for (int w = 0; w < 8; ++w) t += s_w[w];
-            B.scan_part[U.begin / kScanChunk] = t;
-        }
-        __syncthreads();
+    a = __reduce_add_sync(0xffffffffu, a);
+    if ((threadIdx.x & 31) == 0) s_w[threadIdx.x / 32] = a;
+    __syncthreads();
+    int t = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) t += s_w[w];
+    __syncthreads();
+    return t;
+}
+
+template <int SEL> __device__ __forceinline__ void scan_reduce_unit(const BoxDesc &B, const Unit &U, int *s_w)
+{
+    const int ch = U.begin / kScanChunk;
+    if (ch < scan_first<SEL>(B)) return;
+    const int *in = scan_in<SEL>(B);
+    const int n = min(U.end, scan_len<SEL>(B));
+    int a = 0;
+#pragma unroll
+    for (int q = 0; q < kScanChunk / 256; ++q) {
+        const int k = U.begin + q * 256 + (int)threadIdx.x;
+        a += k < n ? in[k] : 0;
     }
+    a = block_sum_256(a, s_w);
+    if (threadIdx.x == 0) scan_part<SEL>(B)[ch] = a;
 }
 
 __device__ __forceinline__ int block_exclusive_scan_256(int v, int *s_w, int &total)
@@ -144,86 +162,106 @@ __device__ __forceinline__ int block_exclusive_scan_256(int v, int *s_w, int &to
     return r;
 }
 
-template <int SEL>
-__global__ void __launch_bounds__(256) k_scan_top(const BoxDesc *__restrict__ boxes, int nbox)
+// PARTS: the chunks before this one come from scan_reduce_unit's sums, else from their counts
+template <int SEL, bool PARTS>
+__device__ __forceinline__ void scan_down_unit(const BoxDesc &B, const Unit &U, int *s_w)
 {
-    __shared__ int s_w[16];
-    const int b = blockIdx.x;
-    if (b >= nbox) return;
-    const BoxDesc &B = boxes[b];
-    if (!rebuilding(B)) return;
-    const int nch = (scan_len<SEL>(B) + kScanChunk - 1) / kScanChunk;
-    int carry = 0;
-    for (int base = 0; base < nch; base += 256) {
-        const int k = base + threadIdx.x;
-        const int v = k < nch ? B.scan_part[k] : 0;
-        int total;
-        const int ex = block_exclusive_scan_256(v, s_w, total);
-        if (k < nch) B.scan_part[k] = carry + ex;
-        carry += total;
+    const int ch = U.begin / kScanChunk, c0 = scan_first<SEL>(B);
+    if (ch < c0) return;
+    const int *in = scan_in<SEL>(B);
+    const int n = scan_len<SEL>(B);
+    // 8 items per thread, blocked
+    int v[8];
+    const int k0 = U.begin + threadIdx.x * 8;
+    int local = 0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        v[q] = (k0 + q < min(U.end, n)) ? in[k0 + q] : 0;
+        local += v[q];
     }
-    if (threadIdx.x == 0) B.scan_part[nch] = carry;
+    int before = 0;
+    if (PARTS) {
+        const int *part = scan_part<SEL>(B);
+        for (int k = c0 + threadIdx.x; k < ch; k += 256) before += part[k];
+    } else {
+        // whole chunks: eight counts per thread and chunk, 16-byte loads (arrays are 256-byte aligned)
+#pragma unroll 4
+        for (int k = c0 * (kScanChunk / 4) + threadIdx.x; k < ch * (kScanChunk / 4); k += 256) {
+            const int4 q = reinterpret_cast<const int4 *>(in)[k];
+            before += q.x + q.y + q.z + q.w;
+        }
+    }
+    const int carry = block_sum_256(before, s_w);
+    int total;
+    int ex = block_exclusive_scan_256(local, s_w, total) + carry;
+    // images past the ghost capacity are counted in their bins but never written: the starts
+    // stay inside the bin-ordered arrays (the box reports the overflow)
+    const int cap = B.nlocal + B.ghost_cap;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const int k = k0 + q;
+        if (k < U.end) {
+            if (SEL == kSelCls) {
+                B.cls_start[k] = ex;
+                B.cls_cursor[k] = ex;
+            } else if (SEL == kSelGhost) {
+                B.gfirst[k] = ex;
+            } else {
+                const int at = min(ex, cap);
+                B.bin_start[k] = at;
+                B.bin_cursor[k] = at;
+            }
+        }
+        ex += v[q];
+    }
+    if (threadIdx.x == 255) {
+        // totals: ghost count / bin_start[nbin] / class sentinel
+        const int tot = ex;
+        if (SEL == kSelGhost && U.end == n + 1) B.st->nghost = tot;
+        if (SEL == kSelBin && U.end == n) B.bin_start[n] = min(tot, cap);
+        if (SEL == kSelCls && U.end == n) B.cls_start[n] = tot;
+    }
 }
 
-template <int SEL>
-__global__ void __launch_bounds__(256) k_scan_down(const BoxDesc *__restrict__ boxes,
-                                                   const Unit *__restrict__ units, int nunits)
+// one or two scans of the same stage: blocks take the units of `a`, then those of `b`.
+// STAGE 0: reduce, 1: down from the reduce's sums, 2: down in one kernel
+template <int SELA, int SELB, int STAGE>
+__global__ void __launch_bounds__(256) k_scan(const BoxDesc *__restrict__ boxes, UnitList a, UnitList b)
 {
     __shared__ int s_w[16];
-    for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
-        const Unit U = units[u];
+    for (int u = blockIdx.x; u < a.n + b.n; u += gridDim.x) {
+        const bool first = u < a.n;
+        const Unit U = first ? a.d[u] : b.d[u - a.n];
         const BoxDesc &B = boxes[U.box];
         if (!rebuilding(B)) continue;
-        int *in = scan_in<SEL>(B);
-        const int n = scan_len<SEL>(B);
-        int carry = B.scan_part[U.begin / kScanChunk];
-        // 8 items per thread, blocked
-        int v[8];
-        const int k0 = U.begin + threadIdx.x * 8;
-        int local = 0;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            v[q] = (k0 + q < U.end) ? in[k0 + q] : 0;
-            local += v[q];
-        }
-        int total;
-        int ex = block_exclusive_scan_256(local, s_w, total) + carry;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const int k = k0 + q;
-            if (k < U.end) {
-                if (SEL == kSelCls) {
-                    B.cls_start[k] = ex;
-                    B.cls_cursor[k] = ex;
-                } else if (SEL == kSelGhost) {
-                    in[k] = ex;
-                } else {
-                    B.bin_start[k] = ex;
-                    B.bin_cursor[k] = ex;
-                }
-            }
-            ex += v[q];
-        }
-        if (U.end == n && threadIdx.x == 255) {
-            // totals: ghost count / bin_start[nbin] / class sentinel
-            const int tot = ex;
-            if (SEL == kSelGhost) B.st->nghost = tot;
-            if (SEL == kSelBin) B.bin_start[n] = tot;
-            if (SEL == kSelCls) B.cls_start[n] = tot;
+        if (STAGE == 0) {
+            if (first) scan_reduce_unit<SELA>(B, U, s_w);
+            else scan_reduce_unit<SELB>(B, U, s_w);
+        } else {
+            if (first) scan_down_unit<SELA, STAGE == 1>(B, U, s_w);
+            else scan_down_unit<SELB, STAGE == 1>(B, U, s_w);
         }
     }
 }
 
 // resident blocks per SM of the scan passes, from the occupancy API (init_rebuild_shapes)
-static int g_scan_reduce[3] = {4, 4, 4}, g_scan_down[3] = {4, 4, 4};
+static int g_scan_cls[3] = {4, 4, 4}, g_scan_bins[3] = {4, 4, 4};
 
-template <int SEL>
-static void scan(cudaStream_t s, BoxDesc *boxes, const UnitList &ul, int nbox, int sms)
+// In one kernel a block adds up every count before its chunk, which costs less than a second
+// launch (~2.5 us) while a scan has up to kShortScan chunks.
+constexpr int kShortScan = 32;
+
+template <int SELA, int SELB>
+static void scan(cudaStream_t s, BoxDesc *boxes, const UnitList &a, const UnitList &b, int longest, int sms,
+                 const int *per_sm)
 {
-    auto g = [&](int per_sm) { return ul.n < sms * per_sm ? (ul.n > 0 ? ul.n : 1) : sms * per_sm; };
-    k_scan_reduce<SEL><<<g(g_scan_reduce[SEL]), 256, 0, s>>>(boxes, ul.d, ul.n);
-    k_scan_top<SEL><<<nbox, 256, 0, s>>>(boxes, nbox);
-    k_scan_down<SEL><<<g(g_scan_down[SEL]), 256, 0, s>>>(boxes, ul.d, ul.n);
+    auto g = [&](int blocks) { return std::max(1, std::min(a.n + b.n, sms * blocks)); };
+    if (longest <= kShortScan) {
+        k_scan<SELA, SELB, 2><<<g(per_sm[2]), 256, 0, s>>>(boxes, a, b);
+    } else {
+        k_scan<SELA, SELB, 0><<<g(per_sm[0]), 256, 0, s>>>(boxes, a, b);
+        k_scan<SELA, SELB, 1><<<g(per_sm[1]), 256, 0, s>>>(boxes, a, b);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -285,7 +323,11 @@ __device__ __forceinline__ void bucket_warp(const BoxDesc &B, int *arr, int s, i
 // each: a bucket of up to 32 members (the usual case: a reorder class is one bin's interior or
 // border locals, ~14 at rho 6.05) is ordered with shuffles inside its group, so the warp waits
 // once for the loads of four buckets; a larger one is ordered by the whole warp afterwards.
+// Work items are 32 buckets (one group of four per warp), so that a small box's few units of 256
+// spread over the chip: with a unit per block each warp took eight groups one after another (the
+// bin pass of a 2,000-particle box: 17.8 us).
 constexpr int kGroupSlots = 4;  // members per lane of an 8-lane group
+constexpr int kBucketItems = 8;
 template <int MODE>  // 0: reorder classes -> perm, 1: bins -> bin_order + bpos
 __global__ void __launch_bounds__(256, 4) k_rb_bucket(const BoxDesc *__restrict__ boxes,
                                                    const Unit *__restrict__ units, int nunits)
@@ -294,20 +336,24 @@ __global__ void __launch_bounds__(256, 4) k_rb_bucket(const BoxDesc *__restrict_
     const int lane = threadIdx.x & 31, w = threadIdx.x / 32;
     const int grp = lane >> 3, l8 = lane & 7;
     unsigned long long *key = s_key[w];
-    for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
-        const Unit U = units[u];
+    for (int it = blockIdx.x; it < nunits * kBucketItems; it += gridDim.x) {
+        const Unit U = units[it / kBucketItems];
         const BoxDesc &B = boxes[U.box];
         if (!rebuilding(B)) continue;
         int *cnt = MODE == 0 ? B.cls_count : B.bin_count;
         const int *start = MODE == 0 ? B.cls_start : B.bin_start;
         int *arr = MODE == 0 ? B.perm : B.bin_order;
         const int lim = MODE == 0 ? B.nlocal : n_all(B);
-        for (int b0 = U.begin + 4 * w; b0 < U.end; b0 += 32) {
+        const int b0 = U.begin + (it % kBucketItems) * 32 + 4 * w;
+        if (b0 < U.end) {
             const int b = b0 + grp;
-            int n = 0, s = 0;
+            int n = 0, s = 0, counted = 0;
             if (b < U.end) {
                 n = cnt[b];
                 s = start[b];
+                // a ghost overflow: the bins' members end with the arrays
+                if (MODE == 1) n = min(n, B.nlocal + B.ghost_cap - s);
+                counted = cnt[b];
             }
             if (n != 0 && !(MDPD_IN(s, s + n) && MDPD_IN(s + n - 1, lim))) {
                 if (l8 == 0) cnt[b] = 0;  // check build: a bucket outside its array
@@ -319,6 +365,7 @@ __global__ void __launch_bounds__(256, 4) k_rb_bucket(const BoxDesc *__restrict_
                 int last = 0;
                 if (n > 0 && l8 == 0) last = arr[s + n - 1];
                 last = __shfl_sync(0xffffffffu, last, grp << 3);
+                if (n == 0 && counted != 0 && l8 == 0) cnt[b] = 0;
                 if (n > 0 && last < B.nlocal) {
                     if (l8 == 0) cnt[b] = 0;
                     n = 0;
@@ -393,6 +440,39 @@ __device__ __forceinline__ int image_mask(const BoxDesc &B, double x, int d)
 
 __device__ __forceinline__ int bits_count(int m) { return 1 + (m & 1) + ((m >> 1) & 1); }
 
+// f(sx, sy, sz) for every periodic image of a particle with image masks m, in the order of the
+// ghost indices: z slowest
+template <class F> __device__ __forceinline__ void for_images(const int m[3], F &&f)
+{
+    for (int sz = -1; sz <= 1; ++sz) {
+        if (sz == 1 && !(m[2] & 1)) continue;
+        if (sz == -1 && !(m[2] & 2)) continue;
+        for (int sy = -1; sy <= 1; ++sy) {
+            if (sy == 1 && !(m[1] & 1)) continue;
+            if (sy == -1 && !(m[1] & 2)) continue;
+            for (int sx = -1; sx <= 1; ++sx) {
+                if (sx == 1 && !(m[0] & 1)) continue;
+                if (sx == -1 && !(m[0] & 2)) continue;
+                if (sx == 0 && sy == 0 && sz == 0) continue;
+                f(sx, sy, sz);
+            }
+        }
+    }
+}
+
+// bin of the image of x shifted by (sx, sy, sz) periods (gpu_assign_bin_id's rule)
+__device__ __forceinline__ int image_bin(const BoxDesc &B, const double x[3], int sx, int sy, int sz)
+{
+    const double gc[3] = {x[0] + sx * B.prd[0], x[1] + sy * B.prd[1], x[2] + sz * B.prd[2]};
+    int bid[3];
+    for (int d = 0; d < 3; ++d) {
+        const double v = gc[d];
+        const int b = clamp_bin(bin_coord(v, B.lo[d], B.bininv[d]), B.mbin[d]);
+        bid[d] = v >= B.lo[d] ? (v <= B.hi[d] ? b : B.mbin[d] - 1) : 0;
+    }
+    return bid[0] + B.mbin[0] * (bid[1] + bid[2] * B.mbin[1]);
+}
+
 template <int STYLE>
 __global__ void __launch_bounds__(kUnit) k_rb_permute(BoxDesc *__restrict__ boxes,
                                                       const Unit *__restrict__ units, int nunits,
@@ -437,17 +517,23 @@ __global__ void __launch_bounds__(kUnit) k_rb_permute(BoxDesc *__restrict__ boxe
                                (float)(x[2] - B.cen[2]), pack_w(B, type, mask));
         const uint32_t sg = STYLE == 0 ? sig_mdpd(tag, sn) : sig_dpd(tag, fvx, fvy, fvz, sn);
         B.vel[k] = make_float4(fvx, fvy, fvz, __uint_as_float(sg));
-        // ghost images of this particle
-        int nimg = 1;
-        for (int d = 0; d < 3; ++d) nimg *= bits_count(image_mask(B, x[d], d));
-        B.gfirst[k] = nimg - 1;
-        if (k == B.nlocal - 1) B.gfirst[B.nlocal] = 0;
+        // ghost images of this particle: their number (for the scan) and their bins' counts
+        int m[3], nimg = 1;
+        for (int d = 0; d < 3; ++d) {
+            m[d] = image_mask(B, x[d], d);
+            nimg *= bits_count(m[d]);
+        }
+        B.cls_of[k] = nimg - 1;
         // bin of the local
         int bid[3];
         for (int d = 0; d < 3; ++d) bid[d] = clamp_bin(bin_coord(x[d], B.lo[d], B.bininv[d]), B.mbin[d]);
         const int bin = bid[0] + B.mbin[0] * (bid[1] + bid[2] * B.mbin[1]);
         B.bin_of[k] = bin;
         warp_add1(B.bin_count, MDPD_IDX(bin, B.nbin));
+        if (nimg > 1)
+            for_images(m, [&](int sx, int sy, int sz) {
+                atomicAdd(&B.bin_count[MDPD_IDX(image_bin(B, x, sx, sy, sz), B.nbin)], 1);
+            });
     }
     __shared__ bool s_last;
     __syncthreads();
@@ -469,19 +555,42 @@ __global__ void __launch_bounds__(kUnit) k_rb_permute(BoxDesc *__restrict__ boxe
 }
 
 // ---------------------------------------------------------------------------
-// R7: ghost images of border particles + their bins
+// R7: locals into their bins, ghost images of the border particles and their bins.  A local's
+// place needs no atomics: the reorder sort left a bin's bulk particles, then its border
+// particles, as two runs of consecutive indices, so its rank in the bin (in index order) follows
+// from the class starts; its packed position goes to bpos as well.  Ghost images take atomic
+// slots after the bin's locals, and the bin sort puts them in index order.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kUnit) k_rb_ghosts(const BoxDesc *__restrict__ boxes,
-                                                     const Unit *__restrict__ units, int nunits)
+// the locals of a bin: its bulk run and its border run
+__device__ __forceinline__ int bin_locals(const BoxDesc &B, int bin)
+{
+    const int rk = B.bin_rank[bin];
+    return B.cls_start[rk + 1] - B.cls_start[rk] + B.cls_start[B.nbin + rk + 1] - B.cls_start[B.nbin + rk];
+}
+
+__global__ void __launch_bounds__(kUnit) k_rb_bins(const BoxDesc *__restrict__ boxes,
+                                                   const Unit *__restrict__ units, int nunits)
 {
     for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
         const Unit U = units[u];
         const BoxDesc &B = boxes[U.box];
         if (!rebuilding(B)) continue;
         const int k = U.begin + threadIdx.x;
-        if (k >= U.end || k < B.st->n_bulk) continue;
-        const int c = B.st->cur;
-        const int g0 = B.gfirst[k], g1 = B.gfirst[k + 1];
+        if (k >= U.end) continue;
+        const int nl = B.nlocal, na = nl + B.ghost_cap;  // na: places in the bin-ordered arrays
+        const int c = B.st->cur, n_bulk = B.st->n_bulk;
+        const int bin = MDPD_IDX(B.bin_of[k], B.nbin);
+        const float4 pk = B.pos[k];
+        const bool edge = k >= n_bulk;
+        const int g0 = edge ? B.gfirst[k] : 0, g1 = edge ? B.gfirst[k + 1] : 0;
+        const int rk = B.bin_rank[bin];
+        const int b0 = B.cls_start[rk], b1 = B.cls_start[rk + 1];  // the bin's bulk run
+        const int e0 = B.cls_start[B.nbin + rk];                     // its border run
+        const int p = MDPD_IDX(B.bin_start[bin] + (edge ? (b1 - b0) + (k - e0) : k - b0), na);
+        if (p < na) {
+            B.bpos[p] = list_pos(pk, k, nl);
+            B.bin_order[p] = k;
+        }
         if (g1 == g0) continue;
         double x[3];
         int m[3];
@@ -490,79 +599,24 @@ __global__ void __launch_bounds__(kUnit) k_rb_ghosts(const BoxDesc *__restrict__
             m[d] = image_mask(B, x[d], d);
         }
         const float4 vk = B.vel[k];
-        const float w = B.pos[k].w;
         int g = g0;
-        for (int sz = -1; sz <= 1; ++sz) {
-            if (sz == 1 && !(m[2] & 1)) continue;
-            if (sz == -1 && !(m[2] & 2)) continue;
-            for (int sy = -1; sy <= 1; ++sy) {
-                if (sy == 1 && !(m[1] & 1)) continue;
-                if (sy == -1 && !(m[1] & 2)) continue;
-                for (int sx = -1; sx <= 1; ++sx) {
-                    if (sx == 1 && !(m[0] & 1)) continue;
-                    if (sx == -1 && !(m[0] & 2)) continue;
-                    if (sx == 0 && sy == 0 && sz == 0) continue;
-                    if (g >= B.ghost_cap) {
-                        atomicOr(&B.st->status, kErrGhostOverflow);
-                        continue;
-                    }
-                    const double gx = x[0] + sx * B.prd[0];
-                    const double gy = x[1] + sy * B.prd[1];
-                    const double gz = x[2] + sz * B.prd[2];
-                    const int gi = B.nlocal + g;
-                    B.gsrc[g] = k;
-                    const int code = (sx + 1) + 3 * (sy + 1) + 9 * (sz + 1);
-                    B.gimg[g] = code;
-                    B.pos[gi] = make_float4((float)(gx - B.cen[0]), (float)(gy - B.cen[1]),
-                                            (float)(gz - B.cen[2]), ghost_w(w, code));
-                    B.vel[gi] = vk;
-                    const double gc[3] = {gx, gy, gz};
-                    int bid[3];
-                    for (int d = 0; d < 3; ++d) {
-                        const double v = gc[d];
-                        const int b = clamp_bin(bin_coord(v, B.lo[d], B.bininv[d]), B.mbin[d]);
-                        bid[d] = v >= B.lo[d] ? (v <= B.hi[d] ? b : B.mbin[d] - 1) : 0;
-                    }
-                    const int bin = bid[0] + B.mbin[0] * (bid[1] + bid[2] * B.mbin[1]);
-                    B.bin_of[gi] = bin;
-                    atomicAdd(&B.bin_count[MDPD_IDX(bin, B.nbin)], 1);
-                    ++g;
-                }
+        for_images(m, [&](int sx, int sy, int sz) {
+            if (g >= B.ghost_cap) {
+                atomicOr(&B.st->status, kErrGhostOverflow);
+                return;
             }
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
-// R9: scatter locals+ghosts into bins.  A local's place needs no atomics: the reorder sort
-// left a bin's bulk particles, then its border particles, as two runs of consecutive indices,
-// so its rank in the bin (in index order) follows from the class starts; its packed position
-// goes to bpos as well.  Ghost images take atomic slots after the bin's locals, and the bin
-// sort puts them in index order.
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kUnit) k_rb_scatter_bins(const BoxDesc *__restrict__ boxes,
-                                                           const Unit *__restrict__ units, int nunits)
-{
-    for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
-        const Unit U = units[u];
-        const BoxDesc &B = boxes[U.box];
-        if (!rebuilding(B)) continue;
-        const int i = U.begin + threadIdx.x;
-        const int nl = B.nlocal;
-        if (i >= U.end || i >= nl + min(B.st->nghost, B.ghost_cap)) continue;
-        const int bin = MDPD_IDX(B.bin_of[i], B.nbin);
-        const int rk = B.bin_rank[bin];
-        const int b0 = B.cls_start[rk], b1 = B.cls_start[rk + 1];  // the bin's bulk run
-        const int e0 = B.cls_start[B.nbin + rk];                     // its border run
-        int p;
-        if (i < nl) {
-            p = MDPD_IDX(B.bin_start[bin] + (i < B.st->n_bulk ? i - b0 : (b1 - b0) + (i - e0)), n_all(B));
-            B.bpos[p] = list_pos(B.pos[i], i, nl);
-        } else {
-            const int nloc = (b1 - b0) + (B.cls_start[B.nbin + rk + 1] - e0);
-            p = MDPD_IDX(warp_add1(B.bin_cursor, bin) + nloc, n_all(B));
-        }
-        B.bin_order[p] = i;
+            const int gi = nl + g;
+            B.gsrc[g] = k;
+            const int code = (sx + 1) + 3 * (sy + 1) + 9 * (sz + 1);
+            B.gimg[g] = code;
+            B.pos[gi] = make_float4((float)(x[0] + sx * B.prd[0] - B.cen[0]), (float)(x[1] + sy * B.prd[1] - B.cen[1]),
+                                    (float)(x[2] + sz * B.prd[2] - B.cen[2]), ghost_w(pk.w, code));
+            B.vel[gi] = vk;
+            const int gb = MDPD_IDX(image_bin(B, x, sx, sy, sz), B.nbin);
+            const int q = MDPD_IDX(bin_locals(B, gb) + atomicAdd(&B.bin_cursor[gb], 1), na);
+            if (q < na) B.bin_order[q] = gi;
+            ++g;
+        });
     }
 }
 
@@ -806,7 +860,7 @@ void launch_bin_ranks(cudaStream_t s, const int mbin[3], int *rank)
 // holds blocks: the grid is the occupancy the registers allow (12 to 16 blocks for the lighter
 // passes), not a fixed 8.
 struct RebuildShapes {
-    int key = 8, cls = 8, permute0 = 8, permute1 = 8, ghosts = 8, bins = 8;
+    int key = 8, cls = 8, permute0 = 8, permute1 = 8, bins = 8;
 };
 static RebuildShapes g_shapes;
 static std::once_flag g_shapes_once;
@@ -828,14 +882,13 @@ void init_rebuild_shapes()
         g_shapes.cls = resident_blocks(k_rb_scatter_cls);
         g_shapes.permute0 = resident_blocks(k_rb_permute<0>);
         g_shapes.permute1 = resident_blocks(k_rb_permute<1>);
-        g_shapes.ghosts = resident_blocks(k_rb_ghosts);
-        g_shapes.bins = resident_blocks(k_rb_scatter_bins);
-        g_scan_reduce[0] = resident_blocks(k_scan_reduce<0>, 256, 4);
-        g_scan_reduce[1] = resident_blocks(k_scan_reduce<1>, 256, 4);
-        g_scan_reduce[2] = resident_blocks(k_scan_reduce<2>, 256, 4);
-        g_scan_down[0] = resident_blocks(k_scan_down<0>, 256, 4);
-        g_scan_down[1] = resident_blocks(k_scan_down<1>, 256, 4);
-        g_scan_down[2] = resident_blocks(k_scan_down<2>, 256, 4);
+        g_shapes.bins = resident_blocks(k_rb_bins);
+        g_scan_cls[0] = resident_blocks(k_scan<kSelCls, kSelCls, 0>, 256, 4);
+        g_scan_cls[1] = resident_blocks(k_scan<kSelCls, kSelCls, 1>, 256, 4);
+        g_scan_cls[2] = resident_blocks(k_scan<kSelCls, kSelCls, 2>, 256, 4);
+        g_scan_bins[0] = resident_blocks(k_scan<kSelGhost, kSelBin, 0>, 256, 4);
+        g_scan_bins[1] = resident_blocks(k_scan<kSelGhost, kSelBin, 1>, 256, 4);
+        g_scan_bins[2] = resident_blocks(k_scan<kSelGhost, kSelBin, 2>, 256, 4);
     });
 }
 
@@ -846,18 +899,16 @@ void launch_rebuild(cudaStream_t s, BoxDesc *boxes, const BatchUnits &u, const S
     const RebuildShapes &r = g_shapes;
     auto g = [&](int n, int per_sm) { return n < sms * per_sm ? (n > 0 ? n : 1) : sms * per_sm; };
     k_rb_key<<<g(u.local.n, r.key), kUnit, 0, s>>>(boxes, u.local.d, u.local.n);
-    scan<kSelCls>(s, boxes, u.scan_cls, u.nbox, sms);
+    scan<kSelCls, kSelCls>(s, boxes, u.scan_cls, UnitList{}, u.longest_cls, sms, g_scan_cls);
     k_rb_scatter_cls<<<g(u.local.n, r.cls), kUnit, 0, s>>>(boxes, u.local.d, u.local.n);
-    k_rb_bucket<0><<<g(u.cls.n, 4), 256, 0, s>>>(boxes, u.cls.d, u.cls.n);
+    k_rb_bucket<0><<<g(u.cls.n * kBucketItems, 4), 256, 0, s>>>(boxes, u.cls.d, u.cls.n);
     if (c.style == 0)
         k_rb_permute<0><<<g(u.local.n, r.permute0), kUnit, 0, s>>>(boxes, u.local.d, u.local.n, u.nbox, done);
     else
         k_rb_permute<1><<<g(u.local.n, r.permute1), kUnit, 0, s>>>(boxes, u.local.d, u.local.n, u.nbox, done);
-    scan<kSelGhost>(s, boxes, u.scan_ghost, u.nbox, sms);
-    k_rb_ghosts<<<g(u.local.n, r.ghosts), kUnit, 0, s>>>(boxes, u.local.d, u.local.n);
-    scan<kSelBin>(s, boxes, u.scan_bin, u.nbox, sms);
-    k_rb_scatter_bins<<<g(u.all.n, r.bins), kUnit, 0, s>>>(boxes, u.all.d, u.all.n);
-    k_rb_bucket<1><<<g(u.bins.n, 4), 256, 0, s>>>(boxes, u.bins.d, u.bins.n);
+    scan<kSelGhost, kSelBin>(s, boxes, u.scan_ghost, u.scan_bin, u.longest_ghost, sms, g_scan_bins);
+    k_rb_bins<<<g(u.local.n, r.bins), kUnit, 0, s>>>(boxes, u.local.d, u.local.n);
+    k_rb_bucket<1><<<g(u.bins.n * kBucketItems, 4), 256, 0, s>>>(boxes, u.bins.d, u.bins.n);
     k_rb_list<<<g(u.bins.n * 32, 4), 256, 0, s>>>(boxes, u.bins.d, u.bins.n, u.nbox, done + 1);
 }
 

@@ -14,12 +14,12 @@ struct UnitList {
 // units of one batch, by domain (all boxes concatenated)
 struct BatchUnits {
     UnitList local;      // [0,nlocal) in chunks of kUnit, 32-aligned
-    UnitList all;        // [0,nlocal+ghost_cap) in chunks of kUnit
     UnitList cls;        // [0,2*nbin) in chunks of 256 buckets
     UnitList bins;       // [0,nbin) in chunks of 256 bins
     UnitList scan_cls;   // [0,2*nbin) in chunks of kScanChunk
     UnitList scan_ghost; // [0,nlocal+1)
     UnitList scan_bin;   // [0,nbin)
+    int longest_cls = 0, longest_ghost = 0;  // chunks of the longest scan: classes; ghosts or bins
     int nbox = 0;
 };
 

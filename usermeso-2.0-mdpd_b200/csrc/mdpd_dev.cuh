@@ -129,14 +129,14 @@ struct BoxDesc {
     // ---- rebuild scratch ----
     int *bin_rank;        // Morton rank of each bin (reorder class order)
     int *cls_count, *cls_start, *cls_cursor;  // 2*nbin
-    int *cls_of;          // class of each local
+    int *cls_of;          // class of each local; after the class scatter, its number of images
     int *sub_of;          // secondary key of each local
     int *perm;            // new -> old
-    int *bin_of;          // bin of locals+ghosts
+    int *bin_of;          // bin of each local
     int *bin_count, *bin_start, *bin_cursor;  // nbin (+1)
     int *bin_order;       // bin-sorted particle indices
     float4 *bpos;         // positions in bin order
-    int *scan_part;       // per-chunk partial sums for scans
+    int *scan_part, *scan_part2;  // per-chunk sums of the class and bin scans; of the ghost scan
     // ---- thermo partials ----
     double *partial;      // per unit thermo partials (kPartialStride doubles)
     BoxState *st;
