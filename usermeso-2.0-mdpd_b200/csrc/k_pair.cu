@@ -1,7 +1,8 @@
 // mDPD pair passes with each pair evaluated once.
 //
 // k_density_rows: one lane per particle row of the list (32 consecutive particles per warp, the
-//   locally transposed table makes each entry index a coalesced warp load), G = 4, 6 or 8
+//   locally transposed table makes each entry index a coalesced warp load; two to eight lanes per
+//   row where the chip is not full, density_lanes), G = 4, 6 or 8
 //   neighbour positions in flight per lane (the batch's autotuner picks G).  rho_i
 //   (fix_aboundary_rho_meso.cu:119-165) is summed in FP32 with the hardware rsqrt, as the
 //   reference forms each term; the reference adds the terms in FP64, which changes rho by about
@@ -138,14 +139,111 @@ template <int kGather, bool UNI> __device__ __forceinline__ void density_rows(co
     }
 }
 
-template <int kGather, bool UNI>
+// The same rows with LPR lanes each (32 / LPR rows per warp): lane s of a row takes entries
+// s, s + LPR, ..., so a row waits for LPR times fewer rounds of loads, and the terms are added in
+// row order through shuffles (every lane of the row forms the whole sum): the same bits as one
+// lane per row.  `first`: first row of the block's 128 / LPR.
+template <int kGather, bool UNI, int LPR>
+__device__ __forceinline__ void density_rows_split(const BoxDesc &B, int first, int end)
+{
+    constexpr int R = 32 / LPR;  // rows per warp: lane = s * R + r
+    static_assert(kGather % 2 == 0 && kGather * LPR <= 64, "two entries at a time; a round within two list lines");
+    const int lane = threadIdx.x & 31, s = lane / R, r = lane % R;
+    const int i = first + (threadIdx.x >> 5) * R + r;
+    const bool live = i < end;
+    const int self = live ? i : first;
+    const int ncol = B.n_col, ncol2 = B.n_col2, nlocal = B.nlocal;
+    const int *row = B.table + ((unsigned)(self & ~31) * (unsigned)ncol + (unsigned)(self & 31));  // entry k at 32 k
+    // the first round's entries are read beside the row length (a row holds at least 32 entries;
+    // those past its length are dropped below)
+    int e[kGather];
+#pragma unroll
+    for (int q = 0; q < kGather; ++q) e[q] = q * LPR + s < ncol ? __ldcs(row + 32 * (q * LPR + s)) : 0;
+    const int c = B.st->cur;
+    const bool in_group = live && (B.mask[c][self] & B.rho_bit);
+    const int n = live ? MDPD_IDX(B.count[self], ncol + 1) : 0;
+    const float4 pi = B.pos[self];
+    const bool edge = live && self >= B.st->n_bulk;
+    const int g0 = edge ? B.gfirst[self] : 0, g1 = edge ? min(B.gfirst[self + 1], B.ghost_cap) : 0;
+    const int nmax = __reduce_max_sync(0xffffffffu, n);
+    const float h = B.cut_rho, rcf2 = B.rc2_force;
+    const unsigned long long pix = pk2(pi.x, pi.x), piy = pk2(pi.y, pi.y), piz = pk2(pi.z, pi.z);
+    const unsigned long long nh = pk2(-h, -h);
+    int *row2 = B.table2 + (size_t)self * ncol2;
+    unsigned mine = 0;  // the lanes of this row
+#pragma unroll
+    for (int q = 0; q < LPR; ++q) mine |= 1u << (q * R);
+    mine <<= r;
+    const unsigned before = mine & ((1u << lane) - 1u);
+    float acc = 0.f;
+    int n2 = 0;
+    for (int k0 = 0; k0 < nmax; k0 += kGather * LPR) {
+        float4 pj[kGather];
+#pragma unroll
+        for (int q = 0; q < kGather; ++q) {
+            const int k = k0 + q * LPR + s;
+            if (k0 != 0) e[q] = k < n ? __ldcs(row + 32 * k) : self;
+            else if (k >= n) e[q] = self;
+        }
+#pragma unroll
+        for (int q = 0; q < kGather; ++q) pj[q] = __ldg(&B.pos[MDPD_IDX(e[q] & kEntryIndexMask, n_all(B))]);
+#pragma unroll
+        for (int q = 0; q < kGather; q += 2) {
+            const unsigned long long dx = sub2(pix, pk2(pj[q].x, pj[q + 1].x));
+            const unsigned long long dy = sub2(piy, pk2(pj[q].y, pj[q + 1].y));
+            const unsigned long long dz = sub2(piz, pk2(pj[q].z, pj[q + 1].z));
+            const unsigned long long rsq = dist2x2(dx, dy, dz);
+            float rr[2], t[2];
+            upk2(rsq, rr[0], rr[1]);
+            upk2(fma2(rsq, pk2(rsqrt_ftz(rr[0]), rsqrt_ftz(rr[1])), nh), t[0], t[1]);
+#pragma unroll
+            for (int h2 = 0; h2 < 2; ++h2) {
+                const float tm = fminf(t[h2], 0.f);
+#pragma unroll
+                for (int q2 = 0; q2 < LPR; ++q2) {
+                    const float tq = __shfl_sync(0xffffffffu, tm, q2 * R + r);
+                    acc = __fmaf_rn(tq, tq, acc);
+                }
+                const int eq = e[q + h2];
+                const bool hit = eq < 0 && rr[h2] < rcf2;
+                const unsigned b = __ballot_sync(0xffffffffu, hit);
+                if (hit) {
+                    const int j = eq & kEntryIndexMask;
+                    row2[min(n2 + __popc(b & before), ncol2 - 1)] = UNI ? j : j | (ptype(pj[q + h2]) << kEntryTypeShift);
+                }
+                n2 += __popc(b & mine);
+            }
+        }
+    }
+    if (live) {
+        const float rho = in_group ? (float)(B.mass[ptype(pi)] * B.rho_factor) * acc : B.rho[i];
+        if (s == 0) {
+            B.count2[i] = min(n2, ncol2);
+            if (n2 > ncol2) atomicOr(&B.st->status, kErrList2Overflow);
+            if (in_group) B.rho[i] = rho;
+            B.posrho[i] = make_float4(pi.x, pi.y, pi.z, rho);
+        }
+        for (int g = g0 + s; g < g1; g += LPR) {
+            if (in_group) B.rho[nlocal + g] = rho;
+            const float4 pg = B.pos[nlocal + g];
+            B.posrho[nlocal + g] = make_float4(pg.x, pg.y, pg.z, rho);
+        }
+    }
+}
+
+template <int kGather, bool UNI, int LPR>
 __global__ void __launch_bounds__(128, density_blocks<kGather>()) k_density_rows(const BoxDesc *__restrict__ boxes,
                                                       const Unit *__restrict__ units, int nunits)
 {
-    const int u = blockIdx.x;
+    const int u = blockIdx.x / LPR;
     if (u >= nunits) return;
     const Unit U = units[u];
-    density_rows<kGather, UNI>(boxes[U.box], U);
+    if (LPR == 1) {
+        density_rows<kGather, UNI>(boxes[U.box], U);
+    } else {
+        const int first = U.begin + (blockIdx.x % LPR) * (128 / LPR);
+        if (first < U.end) density_rows_split<kGather, UNI, LPR == 1 ? 2 : LPR>(boxes[U.box], first, U.end);
+    }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -393,23 +491,48 @@ __global__ void __launch_bounds__(kUnit) k_finalize(const BoxDesc *__restrict__ 
     }
 }
 
+template <int G, bool UNI> static void density_launch(cudaStream_t s, BoxDesc *boxes, const UnitList &u, int lanes)
+{
+    switch (lanes) {
+    case 8: k_density_rows<G, UNI, 8><<<u.n * 8, 128, 0, s>>>(boxes, u.d, u.n); break;
+    case 4: k_density_rows<G, UNI, 4><<<u.n * 4, 128, 0, s>>>(boxes, u.d, u.n); break;
+    case 2: k_density_rows<G, UNI, 2><<<u.n * 2, 128, 0, s>>>(boxes, u.d, u.n); break;
+    default: k_density_rows<G, UNI, 1><<<u.n, 128, 0, s>>>(boxes, u.d, u.n); break;
+    }
+}
+
+template <bool UNI>
+static void density_gather(cudaStream_t s, BoxDesc *boxes, const UnitList &u, int gather, int lanes)
+{
+    switch (gather) {
+    case 4: density_launch<4, UNI>(s, boxes, u, lanes); break;
+    case 8: density_launch<8, UNI>(s, boxes, u, lanes); break;
+    default: density_launch<6, UNI>(s, boxes, u, lanes); break;
+    }
+}
+
+// Lanes per row of the density pass.  A row of ~42 entries takes 7 rounds of 6 gathers, each
+// waiting for its entries and then their positions; while the chip is not full more lanes per row
+// take fewer rounds: the most with which every block is still resident at once (8 per SM), 8
+// lanes only at half of that (most rows are then one round).  With a full chip the shuffles that
+// keep the sum in row order cost more than the rounds saved.  Density pass, us at 1 / 2 / 4 / 8
+// lanes: 2,000 particles 11.7 / 10.3 / 7.9 / 6.4; 8,000 12.0 / 10.2 / 7.8 / 7.8; 20,000 11.9 /
+// 11.5 / 9.9 / 11.5; 42,000 13.8 / 13.0 / 13.0 / 16.4; 100,000 19.6 / 23.1 / 24.4 / 30.4;
+// 200,000 35.9 / 36.7 / 41.5 / 55.0.
+static int density_lanes(int nunits, int sms)
+{
+    const int resident = 8 * sms;
+    if (nunits * 16LL <= resident) return 8;
+    if (nunits * 4LL <= resident) return 4;
+    return nunits * 2LL <= resident ? 2 : 1;
+}
+
 void launch_density_half(cudaStream_t s, BoxDesc *boxes, const BatchUnits &u, const StepConfig &c)
 {
-    const int g = u.local.n;
-    if (g <= 0) return;
-    if (c.uniform_types) {
-        switch (c.gather) {
-        case 4: k_density_rows<4, true><<<g, 128, 0, s>>>(boxes, u.local.d, g); break;
-        case 8: k_density_rows<8, true><<<g, 128, 0, s>>>(boxes, u.local.d, g); break;
-        default: k_density_rows<6, true><<<g, 128, 0, s>>>(boxes, u.local.d, g); break;
-        }
-    } else {
-        switch (c.gather) {
-        case 4: k_density_rows<4, false><<<g, 128, 0, s>>>(boxes, u.local.d, g); break;
-        case 8: k_density_rows<8, false><<<g, 128, 0, s>>>(boxes, u.local.d, g); break;
-        default: k_density_rows<6, false><<<g, 128, 0, s>>>(boxes, u.local.d, g); break;
-        }
-    }
+    if (u.local.n <= 0) return;
+    const int lanes = c.full_chip ? 1 : density_lanes(u.local.n, c.sms);
+    if (c.uniform_types) density_gather<true>(s, boxes, u.local, c.gather, lanes);
+    else density_gather<false>(s, boxes, u.local, c.gather, lanes);
 }
 
 template <bool EXACT, bool EV, bool UNI, int RW>
