@@ -77,3 +77,57 @@ def test_ghost_overflow_is_reported_and_the_library_stays_usable():
     b.step(3)
     assert b.thermo(0).status == 0
     b.close()
+
+
+def deck(n, lo, hi, types, pair, fixes, x, v, style="mdpd"):
+    lam = mdpd.Lammps()
+    lam.commands(f"units lj\nboundary p p p\nneighbor 0.3 bin\nneigh_modify every 1 delay 0 check yes\n"
+                 f"atom_style {style}/atomic/meso 8\n"
+                 f"region box block {lo[0]} {hi[0]} {lo[1]} {hi[1]} {lo[2]} {hi[2]} units box\n"
+                 f"create_box {len(n)} box")
+    for t, c in enumerate(n):
+        lam.command(f"create_atoms {t + 1} random {c} {11 + t} box")
+        lam.command(f"mass {t + 1} 1")
+    lam.commands(types)
+    lam.commands(pair)
+    lam.commands(fixes)
+    lam.commands("timestep 0.01\nrun_style mvv/meso")
+    lam.set_state(x, v)
+    return lam
+
+
+FIELDS = ("tag", "x", "v", "force")
+
+
+def fields(lam, names=FIELDS):
+    return [lam.field(k) for k in names]
+
+
+def same(a, b):
+    return all(np.array_equal(p, q) for p, q in zip(a, b))
+
+
+@pytest.mark.parametrize("exact", ["yes", "no"])
+def test_steps_of_one_run_same_bits_as_single_runs(exact):
+    """12 steps of one call leave each step's final half-kick to the next step; single steps apply
+    it themselves.  One group frozen, one under a body force."""
+    n, L = 3001, 8.0
+    x, v = lattice(n, L, 9)
+    mk = lambda: deck((2000, 1001), (0,) * 3, (L,) * 3,  # noqa: E731
+                      "group mov type 1\ngroup fix type 2",
+                      "pair_style mdpd/meso 1.0 1.0 77\npair_coeff * * -40 25 4.5 1.0 0.75\n"
+                      f"pair_modify rng {'exact' if exact == 'yes' else 'fast'}",
+                      "fix R all aboundary/rho/meso cut_rho 0.75\nfix N mov nve/meso\nfix F mov addforce/meso 0.02 0.0 -0.01",
+                      x, v)
+    a, b = mk(), mk()
+    a.setup()
+    b.setup()
+    a.step(12)
+    for _ in range(12):
+        b.step(1)
+    assert same(fields(a), fields(b))
+    a.run(2)  # a step with energy and virial after deferred ones
+    b.run(2)
+    assert same(fields(a), fields(b))
+    a.close()
+    b.close()

@@ -251,7 +251,7 @@ int mdpd_get_field(mdpd_t *h, const char *name, void *out, int64_t nbytes)
         else if (f == "vel4") get(B.vel, 4);
         else if (f == "rho") get(B.rho, 4);
         else if (f == "force") {  // after post_force, as the reference: pair force + body force
-            get(B.f[c], 4);
+            get(B.f, 4);
             if (B.body_bit) {
                 std::vector<int> mask(cnt / 4);
                 check_cuda(cudaMemcpy(mask.data(), B.mask[c], sizeof(int) * mask.size(), cudaMemcpyDeviceToHost),

@@ -198,10 +198,8 @@ void Box::layout(const Spec &s, int na)
     B.tag[1] = alloc<int>(n);
     B.type[1] = alloc<int>(n);
     B.mask[1] = alloc<int>(n);
-    for (int c = 0; c < 2; ++c) {
-        B.f[c] = alloc<float4>(n);
-        B.phi[c] = alloc<float>(n);
-    }
+    B.f = alloc<float4>(n);
+    for (int c = 0; c < 2; ++c) B.phi[c] = alloc<float>(n);
     B.pos = alloc<float4>(na);
     B.vel = alloc<float4>(na);
     B.rho = alloc<float>(na);
@@ -533,7 +531,7 @@ void Box::download_state(double *x, double *v, double *f, int32_t *tag, int32_t 
     }
     if (f) {
         std::vector<float4> ff(n);
-        check_cuda(cudaMemcpy(ff.data(), desc.f[c], sizeof(float4) * n, cudaMemcpyDeviceToHost), "download");
+        check_cuda(cudaMemcpy(ff.data(), desc.f, sizeof(float4) * n, cudaMemcpyDeviceToHost), "download");
         for (int i = 0; i < n; ++i) {
             f[3 * i] = ff[i].x;
             f[3 * i + 1] = ff[i].y;
@@ -668,7 +666,10 @@ void Batch::capture(int ev)
     check_cuda(cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault), "conditional handle");
     check_cuda(cudaStreamBeginCaptureToGraph(stream_, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal),
                "capture");
-    launch_integrate(stream_, d_boxes, units, cfg, d_done, h, 1);
+    // the plain step leaves its force sums to the next step's integrate (run() ends with a
+    // finalize); the one with energy and virial applies them, as its thermo needs the velocities
+    const bool defer = !ev && defers();
+    launch_integrate(stream_, d_boxes, units, cfg, d_done, h, 1, defer);
     cudaStreamCaptureStatus cs;
     cudaGraph_t cg;
     const cudaGraphNode_t *deps = nullptr;
@@ -691,7 +692,7 @@ void Batch::capture(int ev)
     check_cuda(cudaStreamEndCapture(s2, &tmp), "end body");
     cudaStreamDestroy(s2);
     if (cfg.style == 0) launch_density(stream_, d_boxes, units, cfg);
-    launch_force(stream_, d_boxes, units, cfg, ev, 1);
+    launch_force(stream_, d_boxes, units, cfg, ev, 1, !defer);
     if (cfg.aboundary) launch_aboundary_meso(stream_, d_boxes, units);  // end of step, before output
     if (ev) launch_thermo(stream_, d_boxes, units, d_thermo, d_done + 2);
     check_cuda(cudaStreamEndCapture(stream_, &tmp), "end capture");
@@ -705,7 +706,7 @@ void Batch::setup()
     launch_force_rebuild_flag(stream_, d_boxes, units.nbox, 1);
     launch_rebuild(stream_, d_boxes, units, cfg, d_done);
     if (cfg.style == 0) launch_density(stream_, d_boxes, units, cfg);
-    launch_force(stream_, d_boxes, units, cfg, 1, 0);
+    launch_force(stream_, d_boxes, units, cfg, 1, 0, true);
     launch_force_rebuild_flag(stream_, d_boxes, units.nbox, 0);
     check_cuda(cudaGetLastError(), "setup launch");
     check_cuda(cudaStreamSynchronize(stream_), "setup");
@@ -734,7 +735,7 @@ void Batch::setup_boxes(const std::vector<int> &which)
     const BatchUnits su = make_units(boxes_, which, units.nbox, allocs, stream_);
     launch_rebuild(stream_, d_boxes, su, cfg, d_done);
     if (cfg.style == 0) launch_density(stream_, d_boxes, su, cfg);
-    launch_force(stream_, d_boxes, su, cfg, 1, 0);
+    launch_force(stream_, d_boxes, su, cfg, 1, 0, true);
     launch_force_rebuild_flag(stream_, d_boxes, units.nbox, 0);
     check_cuda(cudaFreeAsync(d, stream_), "setup boxes");
     for (Unit *a : allocs) cudaFreeAsync(a, stream_);
@@ -764,6 +765,10 @@ void Batch::run(long long nsteps, bool sync, bool ev_last)
     Range r("mdpd::run");
     for (long long k = 0; k < nsteps; ++k)
         check_cuda(cudaGraphLaunch(graph_[ev_last && k == nsteps - 1 ? 1 : 0], stream_), "graph launch");
+    if (nsteps > 0 && !ev_last && defers()) {
+        launch_finalize(stream_, d_boxes, units, 1);
+        check_cuda(cudaGetLastError(), "finalize launch");
+    }
     if (sync) check_cuda(cudaStreamSynchronize(stream_), "run");
 }
 
@@ -784,7 +789,7 @@ double Batch::time_pair_passes(int reps)
     check_cuda(cudaEventCreate(&e1), "event");
     auto once = [&] {
         if (cfg.style == 0) launch_density(stream_, d_boxes, units, cfg);
-        launch_force(stream_, d_boxes, units, cfg, 0, 0);
+        launch_force(stream_, d_boxes, units, cfg, 0, 0, true);
     };
     once();
     check_cuda(cudaEventRecord(e0, stream_), "event");
@@ -809,7 +814,7 @@ void Batch::profile(long long nsteps, double out[5])
         cudaEventRecord(ev[0], stream_);
         {
             Range r("integrate");
-            launch_integrate(stream_, d_boxes, units, cfg, d_done, cudaGraphConditionalHandle{}, 0);
+            launch_integrate(stream_, d_boxes, units, cfg, d_done, cudaGraphConditionalHandle{}, 0, false);
         }
         cudaEventRecord(ev[1], stream_);
         {
@@ -824,7 +829,7 @@ void Batch::profile(long long nsteps, double out[5])
         cudaEventRecord(ev[3], stream_);
         {
             Range r("force");
-            launch_force(stream_, d_boxes, units, cfg, 0, 1);
+            launch_force(stream_, d_boxes, units, cfg, 0, 1, true);
             if (cfg.aboundary) launch_aboundary_meso(stream_, d_boxes, units);
         }
         cudaEventRecord(ev[4], stream_);

@@ -174,6 +174,9 @@ private:
     void to_thermo(const double *partials, const BoxState *states, std::vector<Thermo> &out) const;
     void build_units();
     void capture(int ev);
+    // whether a plain step leaves its force sums to the next one (fix aboundary/meso needs v and f
+    // at the end of each step)
+    bool defers() const { return cfg.half && !cfg.aboundary; }
 };
 
 // an NVTX range over a host scope: the phases of setup, stepping, rebuild and I/O show by name on

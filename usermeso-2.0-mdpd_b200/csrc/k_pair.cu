@@ -28,7 +28,8 @@
 //   particle's whole sum inside the fixed-point range; a larger or non-finite term sets the
 //   non-finite status.
 // k_finalize: fixed-point sums -> FP32 pair force, final half-kick (body force added in FP64),
-//   sums cleared.
+//   sums cleared: at the end of a run and of a step with energy and virial.  Between two steps of
+//   a run k_integrate does the same for the step before it, ahead of its own half-kick.
 #include "kernels.h"
 #include "pair.cuh"
 
@@ -38,7 +39,6 @@ namespace mdpd {
 // batch by the autotuner); blocks per SM: 8 at up to 64 registers (G = 4, 6), 7 at up to 72 (G = 8)
 template <int G> constexpr int density_blocks() { return G <= 6 ? 8 : 7; }
 constexpr float kFixF = 4294967296.0f;           // 2^32
-constexpr double kFixInv = 1.0 / 4294967296.0;
 constexpr int kEntryTypeShift = 27;              // compact entry: j | (type of j - 1) << 27
 constexpr int kEntryIndex = (1 << kEntryTypeShift) - 1;
 
@@ -468,6 +468,7 @@ __global__ void __launch_bounds__(kUnit) k_finalize(const BoxDesc *__restrict__ 
         const BoxDesc &B = boxes[U.box];
         const int i = U.begin + threadIdx.x;
         if (i >= U.end) return;
+        if (i == 0) B.st->pending = 0;
         const int c = B.st->cur, n = B.nlocal;
         unsigned long long *fa = B.facc;
         // every load of the particle is issued before the first store (the compiler may not move
@@ -480,8 +481,7 @@ __global__ void __launch_bounds__(kUnit) k_finalize(const BoxDesc *__restrict__ 
         const float fy = (float)((double)ay * kFixInv);
         const float fz = (float)((double)az * kFixInv);
         fa[i] = 0ull, fa[n + i] = 0ull, fa[2 * n + i] = 0ull;
-        if (!(isfinite(fx) && isfinite(fy) && isfinite(fz))) atomicOr(&B.st->status, kErrNonFinite);
-        B.f[c][i] = make_float4(fx, fy, fz, 0.f);  // the pair force; the body force is in the kicks
+        B.f[i] = make_float4(fx, fy, fz, 0.f);  // the pair force; the body force is in the kicks
         if (kick && (m & B.nve_bit)) {
             const bool body = m & B.body_bit;
             B.v[c][0][i] = __fma_rn(dtfm, (double)fx + (body ? B.body[0] : 0.0), vx);
@@ -574,7 +574,8 @@ static void force_half_rows(cudaStream_t s, BoxDesc *boxes, const BatchUnits &u,
     }
 }
 
-void launch_force_half(cudaStream_t s, BoxDesc *boxes, const BatchUnits &u, const StepConfig &c, int ev, int kick)
+void launch_force_half(cudaStream_t s, BoxDesc *boxes, const BatchUnits &u, const StepConfig &c, int ev, int kick,
+                       bool finish)
 {
     const int g = u.local.n;
     if (g <= 0) return;
@@ -590,7 +591,12 @@ void launch_force_half(cudaStream_t s, BoxDesc *boxes, const BatchUnits &u, cons
         if (c.uniform_types) force_half_rows<false, true>(s, boxes, u, rows, staged);
         else force_half_rows<false, false>(s, boxes, u, rows, staged);
     }
-    k_finalize<<<g, kUnit, 0, s>>>(boxes, u.local.d, g, kick);
+    if (finish) launch_finalize(s, boxes, u, kick);
+}
+
+void launch_finalize(cudaStream_t s, BoxDesc *boxes, const BatchUnits &u, int kick)
+{
+    if (u.local.n > 0) k_finalize<<<u.local.n, kUnit, 0, s>>>(boxes, u.local.d, u.local.n, kick);
 }
 
 }  // namespace mdpd

@@ -427,7 +427,8 @@ __global__ void __launch_bounds__(256, 4) k_rb_bucket(const BoxDesc *__restrict_
 }
 
 // ---------------------------------------------------------------------------
-// R5: permute into the other buffer; pack; ghost-image counts; bin the locals
+// R5: permute into the other buffer; pack; ghost-image counts; bin the locals.  The pair force
+// is not carried: integrate has used it, and the force pass after the build writes every one.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ int image_mask(const BoxDesc &B, double x, int d)
 {
@@ -494,9 +495,8 @@ __global__ void __launch_bounds__(kUnit) k_rb_permute(BoxDesc *__restrict__ boxe
             x[d] = B.x[c][d][old];
             v[d] = B.v[c][d][old];
         }
-        const float4 f = B.f[c][old];
         const int tag = B.tag[c][old], type = B.type[c][old], mask = B.mask[c][old];
-        const float phi = B.phi[c][old];
+        const float phi = B.wall_fix ? B.phi[c][old] : 0.f;
         // packed state for the current step (the step counter was advanced by integrate, which
         // left this step's seed in the box state)
         const long long step = S.step;
@@ -507,11 +507,10 @@ __global__ void __launch_bounds__(kUnit) k_rb_permute(BoxDesc *__restrict__ boxe
             B.v[o][d][k] = v[d];
             B.xh[d][k] = x[d];
         }
-        B.f[o][k] = f;
         B.tag[o][k] = tag;
         B.type[o][k] = type;
         B.mask[o][k] = mask;
-        B.phi[o][k] = phi;
+        if (B.wall_fix) B.phi[o][k] = phi;  // zero in both buffers otherwise
         const float fvx = (float)v[0], fvy = (float)v[1], fvz = (float)v[2];
         B.pos[k] = make_float4((float)(x[0] - B.cen[0]), (float)(x[1] - B.cen[1]),
                                (float)(x[2] - B.cen[2]), pack_w(B, type, mask));

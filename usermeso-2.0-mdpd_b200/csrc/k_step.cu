@@ -32,12 +32,14 @@ __device__ __forceinline__ bool last_block(int *done)
 }
 
 // ---------------------------------------------------------------------------
-// integrate: initial half-kick + drift (+ wall bounce-back), displacement check,
-// FP32 pack of locals and their ghost images.  The last block decides the rebuild
+// integrate: (the last step's final half-kick, where its force sums are pending,) initial
+// half-kick + drift (+ wall bounce-back), displacement check, FP32 pack of locals and their ghost images.  The last block decides the rebuild
 // per box (LAMMPS Neighbor::decide) and sets the graph's conditional.
 // ---------------------------------------------------------------------------
-// resident blocks per SM of the integrate pass (the wall variant holds the wall normal sums)
-constexpr int integrate_blocks(bool wall) { return wall ? 5 : 8; }
+// resident blocks per SM of the integrate pass (the wall variant holds the wall normal sums).  7 blocks
+// hold the pending force sums beside the rest in 72 registers; at 8 (64 registers, spills) a 4M box's
+// step takes 2235 us instead of 2210
+constexpr int integrate_blocks(bool wall) { return wall ? 5 : 7; }
 
 // packed position and velocity of ghost g, image `code` of a local at (x, y, z)
 __device__ __forceinline__ void put_ghost(const BoxDesc &B, int g, int code, double x, double y, double z,
@@ -53,7 +55,7 @@ template <bool WALL, int STYLE>
 __global__ void __launch_bounds__(kUnit, integrate_blocks(WALL)) k_integrate(BoxDesc *__restrict__ boxes,
                                                      const Unit *__restrict__ units, int nunits,
                                                      int nbox, int *done,
-                                                     cudaGraphConditionalHandle cond, int use_cond)
+                                                     cudaGraphConditionalHandle cond, int use_cond, int defer)
 {
     for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
         const Unit U = units[u];
@@ -72,7 +74,17 @@ __global__ void __launch_bounds__(kUnit, integrate_blocks(WALL)) k_integrate(Box
             const int t = B.type[c][i], m = B.mask[c][i], tag = B.tag[c][i];
             double x = B.x[c][0][i], y = B.x[c][1][i], z = B.x[c][2][i];
             double vx = B.v[c][0][i], vy = B.v[c][1][i], vz = B.v[c][2][i];
-            const float4 f = B.f[c][i];
+            // the pair force of the last step: from its sums, still to be applied to v, or the array
+            const bool pending = STYLE == 0 && S.pending;
+            long long ax, ay, az;  // the sums, or the bits of the force in FP64
+            if (pending) {
+                const int n = B.nlocal;
+                ax = (long long)B.facc[i], ay = (long long)B.facc[n + i], az = (long long)B.facc[2 * n + i];
+            } else {
+                const float4 f = B.f[i];
+                ax = __double_as_longlong((double)f.x), ay = __double_as_longlong((double)f.y);
+                az = __double_as_longlong((double)f.z);
+            }
             const double hx = B.xh[0][i], hy = B.xh[1][i], hz = B.xh[2][i];
             const bool edge = i >= n_bulk;
             const int g0 = edge ? B.gfirst[i] : 0;
@@ -81,13 +93,24 @@ __global__ void __launch_bounds__(kUnit, integrate_blocks(WALL)) k_integrate(Box
 #pragma unroll
             for (int q = 0; q < 8; ++q) code8[q] = g0 + q < g1 ? B.gimg[g0 + q] : 13;
             const double dtfm = B.dtfm[t - 1];
+            if (pending) {
+                const int n = B.nlocal;
+                ax = __double_as_longlong((double)(float)((double)ax * kFixInv));
+                ay = __double_as_longlong((double)(float)((double)ay * kFixInv));
+                az = __double_as_longlong((double)(float)((double)az * kFixInv));
+                B.facc[i] = 0ull, B.facc[n + i] = 0ull, B.facc[2 * n + i] = 0ull;
+            }
             if (m & B.nve_bit) {
                 // the body force in FP64 (added to FP32 forces it would round the same way for
                 // every particle of a binade: a bias)
                 const bool body = m & B.body_bit;
-                vx = __fma_rn(dtfm, (double)f.x + (body ? B.body[0] : 0.0), vx);
-                vy = __fma_rn(dtfm, (double)f.y + (body ? B.body[1] : 0.0), vy);
-                vz = __fma_rn(dtfm, (double)f.z + (body ? B.body[2] : 0.0), vz);
+                const double fx = __longlong_as_double(ax) + (body ? B.body[0] : 0.0);
+                const double fy = __longlong_as_double(ay) + (body ? B.body[1] : 0.0);
+                const double fz = __longlong_as_double(az) + (body ? B.body[2] : 0.0);
+                if (pending) vx = __fma_rn(dtfm, fx, vx), vy = __fma_rn(dtfm, fy, vy), vz = __fma_rn(dtfm, fz, vz);
+                vx = __fma_rn(dtfm, fx, vx);
+                vy = __fma_rn(dtfm, fy, vy);
+                vz = __fma_rn(dtfm, fz, vz);
                 x = __fma_rn(B.dtv, vx, x);
                 y = __fma_rn(B.dtv, vy, y);
                 z = __fma_rn(B.dtv, vz, z);
@@ -164,26 +187,32 @@ __global__ void __launch_bounds__(kUnit, integrate_blocks(WALL)) k_integrate(Box
     }
     if (last_block(done)) {
         int any = 0;
-        for (int b = threadIdx.x; b < nbox; b += blockDim.x) {
+        // two warps decide, the other two advance the step and its seeds beside them
+        const bool decide = threadIdx.x < kUnit / 2;
+        for (int b = threadIdx.x % (kUnit / 2); b < nbox; b += kUnit / 2) {
             BoxState *S = boxes[b].st;
             const BoxDesc &B = boxes[b];
+            if (!decide) {
+                // this step's seed (for a rebuild's pack) and the next step's, once per box instead
+                // of once per particle (64 TEA rounds)
+                const long long s1 = S->step + 1;
+                const uint32_t used =
+                    S->sn_ok && S->sn_step == s1 && S->sn_seed == B.seed ? S->sn : seed_now(B.seed, s1);
+                S->step = s1;
+                S->sn_prev = used;
+                S->sn = seed_now(B.seed, s1 + 1);
+                S->sn_step = s1 + 1;
+                S->sn_seed = B.seed;
+                S->sn_ok = 1;
+                continue;
+            }
             const int moved = atomicExch(&S->moved, 0);
             const int ago = S->ago + 1;
             int rb = 0;
             if (ago >= B.delay && ago % B.every == 0) rb = B.check ? moved : 1;
             S->rebuild = rb;
             S->ago = rb ? 0 : ago;
-            // this step's seed (for a rebuild's pack) and the next step's, once per box instead
-            // of once per particle (64 TEA rounds)
-            const long long s1 = S->step + 1;
-            const uint32_t used =
-                S->sn_ok && S->sn_step == s1 && S->sn_seed == B.seed ? S->sn : seed_now(B.seed, s1);
-            S->step = s1;
-            S->sn_prev = used;
-            S->sn = seed_now(B.seed, s1 + 1);
-            S->sn_step = s1 + 1;
-            S->sn_seed = B.seed;
-            S->sn_ok = 1;
+            S->pending = defer;
             any |= rb;
         }
         any = __syncthreads_or(any);
@@ -196,21 +225,21 @@ __global__ void __launch_bounds__(kUnit, integrate_blocks(WALL)) k_integrate(Box
 }
 
 void launch_integrate(cudaStream_t s, BoxDesc *boxes, const BatchUnits &u, const StepConfig &c,
-                      int *done, cudaGraphConditionalHandle cond, int use_cond)
+                      int *done, cudaGraphConditionalHandle cond, int use_cond, bool defer)
 {
     const int full = c.sms * integrate_blocks(c.wall);  // one resident wave, grid-stride over units
     int grid = u.local.n < full ? u.local.n : full;
     if (grid < 1) grid = 1;
     if (c.wall) {
         if (c.style == 0)
-            k_integrate<true, 0><<<grid, kUnit, 0, s>>>(boxes, u.local.d, u.local.n, u.nbox, done, cond, use_cond);
+            k_integrate<true, 0><<<grid, kUnit, 0, s>>>(boxes, u.local.d, u.local.n, u.nbox, done, cond, use_cond, defer);
         else
-            k_integrate<true, 1><<<grid, kUnit, 0, s>>>(boxes, u.local.d, u.local.n, u.nbox, done, cond, use_cond);
+            k_integrate<true, 1><<<grid, kUnit, 0, s>>>(boxes, u.local.d, u.local.n, u.nbox, done, cond, use_cond, defer);
     } else {
         if (c.style == 0)
-            k_integrate<false, 0><<<grid, kUnit, 0, s>>>(boxes, u.local.d, u.local.n, u.nbox, done, cond, use_cond);
+            k_integrate<false, 0><<<grid, kUnit, 0, s>>>(boxes, u.local.d, u.local.n, u.nbox, done, cond, use_cond, defer);
         else
-            k_integrate<false, 1><<<grid, kUnit, 0, s>>>(boxes, u.local.d, u.local.n, u.nbox, done, cond, use_cond);
+            k_integrate<false, 1><<<grid, kUnit, 0, s>>>(boxes, u.local.d, u.local.n, u.nbox, done, cond, use_cond, defer);
     }
 }
 
@@ -257,7 +286,7 @@ __global__ void __launch_bounds__(kUnit) k_aboundary_meso(BoxDesc *__restrict__ 
         const float dt = (float)B.dtv;
         const float hs = (float)(0.5 * (double)dt);
         const bool body = m & B.body_bit;
-        const float4 fp = B.f[c][i];
+        const float4 fp = B.f[i];
         // the total force (pair + fix addforce/meso), as the reference's f holds it
         const double fx = (double)fp.x + (body ? B.body[0] : 0.0), fy = (double)fp.y + (body ? B.body[1] : 0.0),
                      fz = (double)fp.z + (body ? B.body[2] : 0.0);
@@ -294,7 +323,7 @@ __global__ void __launch_bounds__(kUnit) k_aboundary_meso(BoxDesc *__restrict__ 
             B.v[c][1][i] = vy - (double)(2.f * vd * ey_);
             B.v[c][2][i] = vz - (double)(2.f * vd * ez_);
             // f keeps the pair force; the body force is added again by the kicks
-            B.f[c][i] = make_float4((float)(fx - (double)(2.f * fd * ex_) - (body ? B.body[0] : 0.0)),
+            B.f[i] = make_float4((float)(fx - (double)(2.f * fd * ex_) - (body ? B.body[0] : 0.0)),
                                     (float)(fy - (double)(2.f * fd * ey_) - (body ? B.body[1] : 0.0)),
                                     (float)(fz - (double)(2.f * fd * ez_) - (body ? B.body[2] : 0.0)), fp.w);
         }
@@ -486,7 +515,7 @@ __global__ void __launch_bounds__(kUnit *TPP, 8 / TPP) k_force(const BoxDesc *__
         if (live && t == 0) {
             const int m = B.mask[c][i];
             if (!(isfinite(fx) && isfinite(fy) && isfinite(fz))) atomicOr(&B.st->status, kErrNonFinite);
-            B.f[c][i] = make_float4(fx, fy, fz, 0.f);  // the pair force; the body force is in the kicks
+            B.f[i] = make_float4(fx, fy, fz, 0.f);  // the pair force; the body force is in the kicks
             if (kick && (m & B.nve_bit)) {
                 const double dtfm = B.dtfm[ptype(pi)];
                 const bool body = m & B.body_bit;
@@ -553,10 +582,11 @@ static void force_launch_style(cudaStream_t s, BoxDesc *boxes, const BatchUnits 
     }
 }
 
-void launch_force(cudaStream_t s, BoxDesc *boxes, const BatchUnits &u, const StepConfig &c, int ev, int kick)
+void launch_force(cudaStream_t s, BoxDesc *boxes, const BatchUnits &u, const StepConfig &c, int ev, int kick,
+                  bool finish)
 {
     if (c.half) {
-        launch_force_half(s, boxes, u, c, ev, kick);
+        launch_force_half(s, boxes, u, c, ev, kick, finish);
         return;
     }
     const int grid = u.local.n < c.sms * 16 ? (u.local.n > 0 ? u.local.n : 1) : c.sms * 16;

@@ -50,18 +50,22 @@ struct Counters {
 };
 
 void launch_integrate(cudaStream_t s, BoxDesc *boxes, const BatchUnits &u, const StepConfig &c,
-                      int *done, cudaGraphConditionalHandle cond, int use_cond);
+                      int *done, cudaGraphConditionalHandle cond, int use_cond, bool defer);
 void launch_force_rebuild_flag(cudaStream_t s, BoxDesc *boxes, int nbox, int value);
 void launch_rebuild(cudaStream_t s, BoxDesc *boxes, const BatchUnits &u, const StepConfig &c,
                     int *done);
 // the rebuild passes' grid sizes from the occupancy API: call once before any stream capture
 void init_rebuild_shapes();
 void launch_density(cudaStream_t s, BoxDesc *boxes, const BatchUnits &u, const StepConfig &c);
+// finish: the pair-once passes end with launch_finalize (without it the sums stay in facc for
+// the next integrate or finalize)
 void launch_force(cudaStream_t s, BoxDesc *boxes, const BatchUnits &u, const StepConfig &c, int ev,
-                  int kick);
+                  int kick, bool finish);
+void launch_finalize(cudaStream_t s, BoxDesc *boxes, const BatchUnits &u, int kick);
 void launch_aboundary_meso(cudaStream_t s, BoxDesc *boxes, const BatchUnits &u);
 void launch_density_half(cudaStream_t s, BoxDesc *boxes, const BatchUnits &u, const StepConfig &c);
-void launch_force_half(cudaStream_t s, BoxDesc *boxes, const BatchUnits &u, const StepConfig &c, int ev, int kick);
+void launch_force_half(cudaStream_t s, BoxDesc *boxes, const BatchUnits &u, const StepConfig &c, int ev, int kick,
+                       bool finish);
 // AoS x[3n] (and v[3n], or zero when null) -> components x[d], xh[d], v[d]; tags 1..n, type 1
 // and mask 1 into the arrays given (null: left as uploaded)
 void launch_load_state(cudaStream_t s, const double *xa, const double *va, int n, double *const x[3],

@@ -55,7 +55,7 @@ struct BoxState {
     int max_count;         // largest neighbour count at the last build
     long long nbuild;
     int cur;               // live copy of the double-buffered arrays
-    int pad;
+    int pending;           // facc holds a force pass's sums that no finalize or integrate has applied
     // seed_now(sn_seed, sn_step) and seed_now(sn_seed, sn_step - 1), computed once per box by
     // the integrate pass of the step before (valid when sn_ok; a host-written state has sn_ok = 0)
     long long sn_step;
@@ -97,7 +97,7 @@ struct BoxDesc {
     // ---- per-particle arrays (locals), double-buffered for the reorder: the live copy
     //      is [st->cur], the other receives the permuted state at a rebuild ----
     double *x[2][3], *v[2][3], *xh[3];
-    float4 *f[2];
+    float4 *f;            // FP32 pair force; written by the end of a step, read by the next one's start
     int *tag[2], *type[2], *mask[2];
     // ---- packed FP32 state, locals then ghosts ----
     float4 *pos, *vel;
@@ -142,6 +142,7 @@ struct BoxDesc {
     BoxState *st;
 };
 
+constexpr double kFixInv = 1.0 / 4294967296.0;  // one unit of the fixed-point force sums
 constexpr int kPartialStride = 18;  // see k_thermo_units for the slot map
 
 // ---------------------------------------------------------------------------
