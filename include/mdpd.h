@@ -56,7 +56,8 @@ typedef struct mdpd_thermo_t {
     double surface_tension; /* (Lx/2)(Pxx - (Pyy+Pzz)/2) for a slab normal to x */
     int32_t status;       /* device error bits: 1 list, 2 ghost, 4 bin/bucket overflow, 8 non-finite
                              force, 16 particle lost, 32 compact list overflow, 64 index out of
-                             range (index-check build) */
+                             range (index-check build), 128 a bounded wait between the blocks of
+                             a run ran out (MDPD_ERR_TIMEOUT) */
     int32_t pad;
 } mdpd_thermo_t;
 

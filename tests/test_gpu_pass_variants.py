@@ -131,3 +131,80 @@ def test_steps_of_one_run_same_bits_as_single_runs(exact):
     assert same(fields(a), fields(b))
     a.close()
     b.close()
+
+
+def wall_box(n_side, exact):
+    """fluid between frozen walls at the low and high x ends"""
+    L = np.array([n_side, 5.0, 5.0])
+    rng = np.random.default_rng(4)
+    nf, nw = int(6.05 * (L[0] - 4) * 25), int(8 * 4 * 25)
+    xf = rng.uniform(0, 1, (nf, 3)) * (L - (4, 0, 0)) + (2, 0, 0)
+    xw = rng.uniform(0, 1, (nw, 3)) * (4, 5, 5)
+    xw[:, 0] = np.mod(xw[:, 0] - 2, L[0])
+    v = np.concatenate([rng.normal(0, 1, (nf, 3)), np.zeros((nw, 3))])
+    return deck((nf, nw), (0,) * 3, L, "group fluid type 1\ngroup solid type 2",
+                "pair_style mdpd/meso 1.0 1.0 77 fluid solid\npair_coeff * * -20 15 4.5 1.0 0.75\n"
+                f"pair_modify rng {exact}",
+                "fix BC all aboundary/rho/meso cut_rho 0.75 phi_c 0.5 cut_phi 1.0 rho_wall 8.0 wall solid mobile fluid\n"
+                "fix NVE fluid nve/meso", np.concatenate([xf, xw]), v)
+
+
+def dpd_box(n, exact):
+    L = (n / 3.0) ** (1 / 3)
+    x, v = lattice(n, L, 6)
+    return deck((n - n // 4, n // 4), (0,) * 3, (L,) * 3, "group all2 type 2",
+                "pair_style dpd/meso 1.0 77\npair_coeff 1 1 25 4.5 3.0 1.0 1.0\npair_coeff 1 2 30 4.5 3.0 1.0 0.9\n"
+                f"pair_coeff 2 2 20 4.5 3.0 1.0 1.0\npair_modify rng {exact}", "fix NVE all nve/meso", x, v, "dpd")
+
+
+def mdpd_box(n, exact):
+    L = (n / RHO) ** (1 / 3)
+    x, v = lattice(n, L, 8)
+    return deck((n - n // 4, n // 4), (0,) * 3, (L,) * 3, "group one type 1",
+                "pair_style mdpd/meso 1.0 1.0 77\npair_coeff 1 1 -40 25 4.5 1.0 0.75\n"
+                "pair_coeff 1 2 -35 25 4.5 0.9 0.7\npair_coeff 2 2 -45 25 4.5 1.0 0.75\n"
+                f"pair_modify rng {exact}",
+                "fix R all aboundary/rho/meso cut_rho 0.75\nfix N all nve/meso\nfix F one addforce/meso 0.02 0.0 -0.01", x, v)
+
+
+# one block per SM holds 1/148 of the rows: boxes at the edges of the lanes-per-row ranges (24 and 96
+# rows per block on a B200), below and above one row per block, and past the run kernel's range
+@pytest.mark.parametrize("exact", ["fast", "exact"])
+@pytest.mark.parametrize("n", [401, 3552, 3553, 14208, 14209, 30011, 70001])
+@pytest.mark.parametrize("make", [mdpd_box, dpd_box])
+def test_runs_of_a_small_box_same_bits_as_step_by_step(make, n, exact):
+    """without thermo output the steps of a run go in one launch; a thermo line at every step makes
+    each a launch of its passes (with energy and virial).  Rebuilds, types, groups, a body force."""
+    a, b = make(n, exact), make(n, exact)
+    b.command("thermo 1")
+    steps = 270 if n < 1000 else 14  # past one launch's 256 steps
+    a.run(steps)
+    b.run(steps)
+    assert a.thermo().nbuild == b.thermo().nbuild >= 3
+    assert same(fields(a, FIELDS + ("rho",)), fields(b, FIELDS + ("rho",)))
+    assert same(a.list_rows(), b.list_rows())
+    a.step(3)
+    for _ in range(3):
+        b.step(1)
+    assert same(fields(a), fields(b))
+    ta, tb = a.thermo(), b.thermo()
+    assert (ta.step, ta.temp, ta.status) == (tb.step, tb.temp, 0)
+    a.close()
+    b.close()
+
+
+def test_one_type_boxes_alone_same_bits_as_in_a_batch():
+    for style, n, kw in ((0, 2500, {}), (0, 20011, dict(exact_rng=1)), (1, 3000, dict(A=25.0, rho_est=0.0)),
+                         (1, 20011, dict(A=25.0, rho_est=0.0, exact_rng=1))):
+        L = (n / (RHO if style == 0 else 3.0)) ** (1 / 3)
+        x, v = lattice(n, L, 3)
+        spec = mdpd.box_spec(n, L, style=style, x=x, v=v, seed=9, **kw)
+        one, two = mdpd.Batch([spec]), mdpd.Batch([spec, spec])
+        for b in (one, two):
+            b.setup()
+            b.step(25)
+            b.step(6)
+        assert all(np.array_equal(p, q) for p, q in zip(one.state(0), two.state(1)))
+        assert one.thermo(0).nbuild == two.thermo(1).nbuild and one.rebuild_steps() == two.rebuild_steps()
+        one.close()
+        two.close()

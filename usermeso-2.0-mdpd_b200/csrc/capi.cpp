@@ -129,7 +129,7 @@ int mdpd_step(mdpd_t *h, int64_t nsteps)
         if (!b || !h->script->box()) throw ScriptError(MDPD_ERR_STATE, "mdpd_step before mdpd_setup/mdpd_run");
         b->run(nsteps, true);
         std::string msg;
-        if (int st = b->status(msg)) throw ScriptError(st & kErrNonFinite ? MDPD_ERR_NAN : MDPD_ERR_OVERFLOW, msg);
+        if (int st = b->status(msg)) throw ScriptError(status_code(st), msg);
     });
 }
 
@@ -467,7 +467,7 @@ int mdpd_batch_setup(mdpd_batch_t *b)
     return guard(b->err, [&] {
         b->batch->setup();
         std::string msg;
-        if (int st = b->batch->status(msg)) throw ScriptError(st & kErrNonFinite ? MDPD_ERR_NAN : MDPD_ERR_OVERFLOW, msg);
+        if (int st = b->batch->status(msg)) throw ScriptError(status_code(st), msg);
     });
 }
 
@@ -477,7 +477,7 @@ int mdpd_batch_step(mdpd_batch_t *b, int64_t nsteps)
     return guard(b->err, [&] {
         b->batch->run(nsteps, true, true);
         std::string msg;
-        if (int st = b->batch->status(msg)) throw ScriptError(st & kErrNonFinite ? MDPD_ERR_NAN : MDPD_ERR_OVERFLOW, msg);
+        if (int st = b->batch->status(msg)) throw ScriptError(status_code(st), msg);
     });
 }
 
@@ -494,7 +494,7 @@ int mdpd_batch_run_thermo(mdpd_batch_t *b, int64_t nsteps, mdpd_thermo_t *out, i
             }
         });
         if (d2h_bytes_per_step) *d2h_bytes_per_step = (int64_t)b->batch->thermo_bytes_per_step();
-        if (bad) throw ScriptError(bad & kErrNonFinite ? MDPD_ERR_NAN : MDPD_ERR_OVERFLOW, status_text(bad));
+        if (bad) throw ScriptError(status_code(bad), status_text(bad));
     });
 }
 
@@ -564,7 +564,7 @@ int mdpd_batch_time(mdpd_batch_t *b, int64_t nsteps, double *ms)
         cudaEventDestroy(e1);
         *ms = t / nsteps;
         std::string msg;
-        if (int st = b->batch->status(msg)) throw ScriptError(st & kErrNonFinite ? MDPD_ERR_NAN : MDPD_ERR_OVERFLOW, msg);
+        if (int st = b->batch->status(msg)) throw ScriptError(status_code(st), msg);
     });
 }
 
@@ -658,7 +658,7 @@ int mdpd_batch_tune(mdpd_batch_t *b, int32_t *shape_density, int32_t *shape_forc
         if (shape_density) *shape_density = p.density;
         if (shape_force) *shape_force = p.force;
         std::string msg;
-        if (int st = b->batch->status(msg)) throw ScriptError(st & kErrNonFinite ? MDPD_ERR_NAN : MDPD_ERR_OVERFLOW, msg);
+        if (int st = b->batch->status(msg)) throw ScriptError(status_code(st), msg);
     });
 }
 
@@ -694,7 +694,7 @@ int mdpd_batch_tune_cached(mdpd_batch_t *b, const char *path, int32_t *shape_den
         if (shape_force) *shape_force = p.force;
         if (cached) *cached = hit ? 1 : 0;
         std::string msg;
-        if (int st = b->batch->status(msg)) throw ScriptError(st & kErrNonFinite ? MDPD_ERR_NAN : MDPD_ERR_OVERFLOW, msg);
+        if (int st = b->batch->status(msg)) throw ScriptError(status_code(st), msg);
     });
 }
 
@@ -753,7 +753,7 @@ int mdpd_batch_profile(mdpd_batch_t *b, int64_t nsteps, double *out5)
     return guard(b->err, [&] {
         b->batch->profile(nsteps, out5);
         std::string msg;
-        if (int st = b->batch->status(msg)) throw ScriptError(st & kErrNonFinite ? MDPD_ERR_NAN : MDPD_ERR_OVERFLOW, msg);
+        if (int st = b->batch->status(msg)) throw ScriptError(status_code(st), msg);
     });
 }
 

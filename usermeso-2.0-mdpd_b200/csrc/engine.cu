@@ -581,6 +581,7 @@ Batch::Batch(std::vector<Box *> boxes, const StepConfig &c) : cfg(c), boxes_(std
         h[b].list_reduce = cfg.half && !cfg.wall && !h[b].wall_fix && !h[b].ab_mobile_bit &&
                            h[b].rn2_list < h[b].rc2_tail;
     }
+    one_ = h[0];
     check_cuda(cudaMemcpyAsync(d_boxes, h.data(), sizeof(BoxDesc) * nb, cudaMemcpyHostToDevice, stream_), "boxes");
     d_done = batch_alloc<int>(4, stream_);
     check_cuda(cudaMemsetAsync(d_done, 0, sizeof(int) * 4, stream_), "done");
@@ -588,7 +589,8 @@ Batch::Batch(std::vector<Box *> boxes, const StepConfig &c) : cfg(c), boxes_(std
     d_states = batch_alloc<BoxState>(nb, stream_);
     build_units();  // synchronises the stream: h, the units and the counters are in place
     init_rebuild_shapes();  // occupancy queries stay out of the captures
-    capture(0);
+    plan_small();
+    if (!small_.kernel) capture(0);
     capture(1);
 }
 
@@ -601,7 +603,7 @@ Batch::~Batch()
     // stream-ordered: after every kernel this batch queued; the stream is released once its
     // work is done
     for (Unit *u : unit_allocs_) cudaFreeAsync(u, stream_);
-    for (void *p : {(void *)d_boxes, (void *)d_done, (void *)d_thermo, (void *)d_states})
+    for (void *p : {(void *)d_boxes, (void *)d_done, (void *)d_thermo, (void *)d_states, (void *)d_bar_})
         if (p) cudaFreeAsync(p, stream_);
     if (h_stage_) cudaFreeHost(h_stage_);
     for (auto &e : ev_stage_)
@@ -756,19 +758,40 @@ void Batch::reconfigure(const StepConfig &c)
     cfg = c;
     cfg.uniform_types = uni;
     cfg.half = half;
-    capture(0);
+    plan_small();
+    if (!small_.kernel) capture(0);
     capture(1);
+}
+
+void Batch::plan_small()
+{
+    small_ = SmallPlan();
+    if (boxes_.size() != 1 || !small_run_plan(one_, cfg, small_)) small_.kernel = nullptr;
+    if (small_.kernel && !d_bar_) d_bar_ = batch_alloc<char>(small_bar_bytes(), stream_);
 }
 
 void Batch::run(long long nsteps, bool sync, bool ev_last)
 {
     Range r("mdpd::run");
-    for (long long k = 0; k < nsteps; ++k)
-        check_cuda(cudaGraphLaunch(graph_[ev_last && k == nsteps - 1 ? 1 : 0], stream_), "graph launch");
-    if (nsteps > 0 && !ev_last && defers()) {
-        launch_finalize(stream_, d_boxes, units, 1);
-        check_cuda(cudaGetLastError(), "finalize launch");
+    const long long plain = nsteps - (ev_last && nsteps > 0 ? 1 : 0);
+    if (small_.kernel) {
+        const cudaError_t e = launch_small_run(stream_, one_, small_, d_bar_, d_done, plain);
+        if (e == cudaErrorCooperativeLaunchTooLarge) {  // part of the device is taken (MPS): nothing was launched
+            (void)cudaGetLastError();
+            small_.kernel = nullptr;
+            capture(0);
+        } else {
+            check_cuda(e, "run launch");
+        }
     }
+    if (!small_.kernel) {
+        for (long long k = 0; k < plain; ++k) check_cuda(cudaGraphLaunch(graph_[0], stream_), "graph launch");
+        if (plain == nsteps && nsteps > 0 && defers()) {
+            launch_finalize(stream_, d_boxes, units, 1);
+            check_cuda(cudaGetLastError(), "finalize launch");
+        }
+    }
+    if (plain < nsteps) check_cuda(cudaGraphLaunch(graph_[1], stream_), "graph launch");
     if (sync) check_cuda(cudaStreamSynchronize(stream_), "run");
 }
 
@@ -969,9 +992,9 @@ std::string status_text(int bits)
 {
     static const char *names[] = {"neighbour list overflow", "ghost capacity overflow", "bin/bucket overflow",
                                   "non-finite force", "particle lost", "compact list overflow",
-                                  "index out of range (index-check build)"};
+                                  "index out of range (index-check build)", "bounded wait ran out"};
     std::string t;
-    for (int k = 0; k < 7; ++k)
+    for (int k = 0; k < 8; ++k)
         if (bits & (1 << k)) t += (t.empty() ? "" : ", ") + std::string(names[k]);
     return t;
 }

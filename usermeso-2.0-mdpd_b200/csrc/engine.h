@@ -164,6 +164,9 @@ private:
     std::vector<Box *> boxes_;
     cudaStream_t stream_ = nullptr;
     int *d_done = nullptr;
+    BoxDesc one_;                  // a single box's descriptor as the passes see it
+    SmallPlan small_;              // its whole-run launch (kernel: null when the box takes the graphs)
+    char *d_bar_ = nullptr;
     double *d_thermo = nullptr;
     BoxState *d_states = nullptr;  // gathered copies of the boxes' scalars
     std::vector<Unit *> unit_allocs_;
@@ -173,6 +176,7 @@ private:
     cudaEvent_t ev_stage_[2] = {nullptr, nullptr};
     void to_thermo(const double *partials, const BoxState *states, std::vector<Thermo> &out) const;
     void build_units();
+    void plan_small();
     void capture(int ev);
     // whether a plain step leaves its force sums to the next one (fix aboundary/meso needs v and f
     // at the end of each step)

@@ -32,27 +32,17 @@
 //   a run k_integrate does the same for the step before it, ahead of its own half-kick.
 #include "kernels.h"
 #include "pair.cuh"
+#include "pair_rows.cuh"
 
 namespace mdpd {
 
 // the density pass keeps G neighbour positions in flight per lane (G = 4, 6 or 8, chosen per
 // batch by the autotuner); blocks per SM: 8 at up to 64 registers (G = 4, 6), 7 at up to 72 (G = 8)
 template <int G> constexpr int density_blocks() { return G <= 6 ? 8 : 7; }
-constexpr float kFixF = 4294967296.0f;           // 2^32
-constexpr int kEntryTypeShift = 27;              // compact entry: j | (type of j - 1) << 27
-constexpr int kEntryIndex = (1 << kEntryTypeShift) - 1;
 
 // ---------------------------------------------------------------------------------------------
 // density pass, global indices
 // ---------------------------------------------------------------------------------------------
-// approximate 1/sqrt(x), denormal inputs taken as 0 (which gives +inf)
-__device__ __forceinline__ float rsqrt_ftz(float x)
-{
-    float y;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
 // One lane per row; the geometry of entries goes two at a time through the two-lane FP32
 // instructions.  A term is (h - r)^2 with r = rsq * rsqrt(rsq), formed as t = rsq * rsqrt(rsq) - h
 // (one rounding; t is -(h - r) exactly) and min(t, 0)^2: pairs beyond the cutoff add 0, and so
@@ -139,98 +129,6 @@ template <int kGather, bool UNI> __device__ __forceinline__ void density_rows(co
     }
 }
 
-// The same rows with LPR lanes each (32 / LPR rows per warp): lane s of a row takes entries
-// s, s + LPR, ..., so a row waits for LPR times fewer rounds of loads, and the terms are added in
-// row order through shuffles (every lane of the row forms the whole sum): the same bits as one
-// lane per row.  `first`: first row of the block's 128 / LPR.
-template <int kGather, bool UNI, int LPR>
-__device__ __forceinline__ void density_rows_split(const BoxDesc &B, int first, int end)
-{
-    constexpr int R = 32 / LPR;  // rows per warp: lane = s * R + r
-    static_assert(kGather % 2 == 0 && kGather * LPR <= 64, "two entries at a time; a round within two list lines");
-    const int lane = threadIdx.x & 31, s = lane / R, r = lane % R;
-    const int i = first + (threadIdx.x >> 5) * R + r;
-    const bool live = i < end;
-    const int self = live ? i : first;
-    const int ncol = B.n_col, ncol2 = B.n_col2, nlocal = B.nlocal;
-    const int *row = B.table + ((unsigned)(self & ~31) * (unsigned)ncol + (unsigned)(self & 31));  // entry k at 32 k
-    // the first round's entries are read beside the row length (a row holds at least 32 entries;
-    // those past its length are dropped below)
-    int e[kGather];
-#pragma unroll
-    for (int q = 0; q < kGather; ++q) e[q] = q * LPR + s < ncol ? __ldcs(row + 32 * (q * LPR + s)) : 0;
-    const int c = B.st->cur;
-    const bool in_group = live && (B.mask[c][self] & B.rho_bit);
-    const int n = live ? MDPD_IDX(B.count[self], ncol + 1) : 0;
-    const float4 pi = B.pos[self];
-    const bool edge = live && self >= B.st->n_bulk;
-    const int g0 = edge ? B.gfirst[self] : 0, g1 = edge ? min(B.gfirst[self + 1], B.ghost_cap) : 0;
-    const int nmax = __reduce_max_sync(0xffffffffu, n);
-    const float h = B.cut_rho, rcf2 = B.rc2_force;
-    const unsigned long long pix = pk2(pi.x, pi.x), piy = pk2(pi.y, pi.y), piz = pk2(pi.z, pi.z);
-    const unsigned long long nh = pk2(-h, -h);
-    int *row2 = B.table2 + (size_t)self * ncol2;
-    unsigned mine = 0;  // the lanes of this row
-#pragma unroll
-    for (int q = 0; q < LPR; ++q) mine |= 1u << (q * R);
-    mine <<= r;
-    const unsigned before = mine & ((1u << lane) - 1u);
-    float acc = 0.f;
-    int n2 = 0;
-    for (int k0 = 0; k0 < nmax; k0 += kGather * LPR) {
-        float4 pj[kGather];
-#pragma unroll
-        for (int q = 0; q < kGather; ++q) {
-            const int k = k0 + q * LPR + s;
-            if (k0 != 0) e[q] = k < n ? __ldcs(row + 32 * k) : self;
-            else if (k >= n) e[q] = self;
-        }
-#pragma unroll
-        for (int q = 0; q < kGather; ++q) pj[q] = __ldg(&B.pos[MDPD_IDX(e[q] & kEntryIndexMask, n_all(B))]);
-#pragma unroll
-        for (int q = 0; q < kGather; q += 2) {
-            const unsigned long long dx = sub2(pix, pk2(pj[q].x, pj[q + 1].x));
-            const unsigned long long dy = sub2(piy, pk2(pj[q].y, pj[q + 1].y));
-            const unsigned long long dz = sub2(piz, pk2(pj[q].z, pj[q + 1].z));
-            const unsigned long long rsq = dist2x2(dx, dy, dz);
-            float rr[2], t[2];
-            upk2(rsq, rr[0], rr[1]);
-            upk2(fma2(rsq, pk2(rsqrt_ftz(rr[0]), rsqrt_ftz(rr[1])), nh), t[0], t[1]);
-#pragma unroll
-            for (int h2 = 0; h2 < 2; ++h2) {
-                const float tm = fminf(t[h2], 0.f);
-#pragma unroll
-                for (int q2 = 0; q2 < LPR; ++q2) {
-                    const float tq = __shfl_sync(0xffffffffu, tm, q2 * R + r);
-                    acc = __fmaf_rn(tq, tq, acc);
-                }
-                const int eq = e[q + h2];
-                const bool hit = eq < 0 && rr[h2] < rcf2;
-                const unsigned b = __ballot_sync(0xffffffffu, hit);
-                if (hit) {
-                    const int j = eq & kEntryIndexMask;
-                    row2[min(n2 + __popc(b & before), ncol2 - 1)] = UNI ? j : j | (ptype(pj[q + h2]) << kEntryTypeShift);
-                }
-                n2 += __popc(b & mine);
-            }
-        }
-    }
-    if (live) {
-        const float rho = in_group ? (float)(B.mass[ptype(pi)] * B.rho_factor) * acc : B.rho[i];
-        if (s == 0) {
-            B.count2[i] = min(n2, ncol2);
-            if (n2 > ncol2) atomicOr(&B.st->status, kErrList2Overflow);
-            if (in_group) B.rho[i] = rho;
-            B.posrho[i] = make_float4(pi.x, pi.y, pi.z, rho);
-        }
-        for (int g = g0 + s; g < g1; g += LPR) {
-            if (in_group) B.rho[nlocal + g] = rho;
-            const float4 pg = B.pos[nlocal + g];
-            B.posrho[nlocal + g] = make_float4(pg.x, pg.y, pg.z, rho);
-        }
-    }
-}
-
 template <int kGather, bool UNI, int LPR>
 __global__ void __launch_bounds__(128, density_blocks<kGather>()) k_density_rows(const BoxDesc *__restrict__ boxes,
                                                       const Unit *__restrict__ units, int nunits)
@@ -242,34 +140,16 @@ __global__ void __launch_bounds__(128, density_blocks<kGather>()) k_density_rows
         density_rows<kGather, UNI>(boxes[U.box], U);
     } else {
         const int first = U.begin + (blockIdx.x % LPR) * (128 / LPR);
-        if (first < U.end) density_rows_split<kGather, UNI, LPR == 1 ? 2 : LPR>(boxes[U.box], first, U.end);
+        const BoxDesc &B = boxes[U.box];
+        const int i0 = first + (threadIdx.x >> 5) * (32 / LPR);
+        if (i0 < U.end)
+            density_rows_split<kGather, UNI, LPR == 1 ? 2 : LPR, false>(B, i0, U.end, B.st->cur, B.st->n_bulk);
     }
 }
 
 // ---------------------------------------------------------------------------------------------
 // force pass
 // ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ long long to_fix(float v) { return __float2ll_rn(v * kFixF); }
-
-// 64-bit fixed-point add into a shared (lo, hi) pair of 32-bit words with native 32-bit
-// atomics: the low word's wrap-arounds carry into the high word, so the pair ends as the exact
-// 64-bit sum (mod 2^64) whatever the order of the adds
-__device__ __forceinline__ void sadd64(unsigned *lo, unsigned *hi, long long q)
-{
-    const unsigned ql = (unsigned)q, qh = (unsigned)((unsigned long long)q >> 32);
-    const unsigned old = atomicAdd(lo, ql);
-    atomicAdd(hi, qh + (old + ql < old ? 1u : 0u));
-}
-
-__device__ __forceinline__ unsigned long long join64(unsigned lo, unsigned hi)
-{
-    return ((unsigned long long)hi << 32) | lo;
-}
-
-// compact entries a warp stages in shared memory per row: rows hold 12.6 owned force-range pairs
-// at rho 6.05; a warp with more than RW times this reads them from the table
-constexpr int kRowEntries = 20;
-
 // shared memory of the force pass, RW rows per warp
 template <int RW> struct RowsSmem {
     PairCoeff coeff[kMaxTypes * kMaxTypes];
@@ -280,29 +160,6 @@ template <int RW> struct RowsSmem {
     double red[4][7];
     int ent[4][RW * kRowEntries];  // each warp's concatenated compact rows (when they fit)
 };
-
-// the warp's rows as one list of T entries split into 32 equal shares; P: prefix of the row
-// lengths (P[r] entries before row r, P[32] = T; len is 0 in lanes that hold no row)
-__device__ __forceinline__ void warp_prefix(int len, int lane, int *P)
-{
-    int pre = len;
-    for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, pre, o);
-        if (lane >= o) pre += v;
-    }
-    P[lane + 1] = pre;
-    if (lane == 0) P[0] = 0;
-}
-
-// the row (of RW) holding entry m of the concatenated rows: the last r with P[r] <= m
-template <int RW> __device__ __forceinline__ int row_of(const int *P, int m)
-{
-    int r = 0;
-#pragma unroll
-    for (int st = RW / 2; st > 0; st >>= 1)
-        if (P[r + st] <= m) r += st;
-    return r;
-}
 
 template <bool EV>
 __device__ __forceinline__ void ev_to_partial(const BoxDesc &B, const Unit &U, const EvAcc &ev, double (*red)[7])

@@ -41,16 +41,6 @@ __device__ __forceinline__ bool last_block(int *done)
 // step takes 2235 us instead of 2210
 constexpr int integrate_blocks(bool wall) { return wall ? 5 : 7; }
 
-// packed position and velocity of ghost g, image `code` of a local at (x, y, z)
-__device__ __forceinline__ void put_ghost(const BoxDesc &B, int g, int code, double x, double y, double z,
-                                          float w, float4 vv)
-{
-    B.pos[B.nlocal + g] = make_float4((float)(x + (code % 3 - 1) * B.prd[0] - B.cen[0]),
-                                      (float)(y + ((code / 3) % 3 - 1) * B.prd[1] - B.cen[1]),
-                                      (float)(z + (code / 9 - 1) * B.prd[2] - B.cen[2]), ghost_w(w, code));
-    B.vel[B.nlocal + g] = vv;
-}
-
 template <bool WALL, int STYLE>
 __global__ void __launch_bounds__(kUnit, integrate_blocks(WALL)) k_integrate(BoxDesc *__restrict__ boxes,
                                                      const Unit *__restrict__ units, int nunits,

@@ -24,6 +24,7 @@ enum : int {
     kErrNonFinite = 8,      // NaN/Inf force
     kErrLost = 16,          // particle outside the box by more than one period
     kErrList2Overflow = 32, // more force-range neighbours than the compact list holds
+    kErrTimeout = 128,      // a bounded wait between the blocks of a run ran out
     kErrIndex = 64,         // check build: an index outside its array (the access was skipped)
 };
 
@@ -519,6 +520,16 @@ constexpr int kUpperImage = 4;
 __device__ __forceinline__ float ghost_w(float w, int code)
 {
     return code > 13 ? __int_as_float(__float_as_int(w) | (kUpperImage << 8)) : w;
+}
+
+// packed position and velocity of ghost g, image `code` of a local at (x, y, z)
+__device__ __forceinline__ void put_ghost(const BoxDesc &B, int g, int code, double x, double y, double z,
+                                          float w, float4 vv)
+{
+    B.pos[B.nlocal + g] = make_float4((float)(x + (code % 3 - 1) * B.prd[0] - B.cen[0]),
+                                      (float)(y + ((code / 3) % 3 - 1) * B.prd[1] - B.cen[1]),
+                                      (float)(z + (code / 9 - 1) * B.prd[2] - B.cen[2]), ghost_w(w, code));
+    B.vel[B.nlocal + g] = vv;
 }
 
 // packed .w word of a position: type-1 in bits 0-7, mobile bit 8, wall bit 9 (bit 10 on ghosts:

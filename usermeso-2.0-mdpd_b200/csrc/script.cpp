@@ -918,7 +918,7 @@ void Script::setup()
     batch_->setup();
     std::string msg;
     const int st = batch_->status(msg);
-    if (st) throw ScriptError(st & kErrNonFinite ? MDPD_ERR_NAN : MDPD_ERR_OVERFLOW, msg);
+    if (st) throw ScriptError(status_code(st), msg);
 }
 
 void Script::thermo(Thermo &t)
@@ -1105,7 +1105,7 @@ void Script::run(long long nsteps)
     batch_->setup();
     step_ = box_->state().step;
     std::string msg;
-    if (int st = batch_->status(msg)) throw ScriptError(st & kErrNonFinite ? MDPD_ERR_NAN : MDPD_ERR_OVERFLOW, msg);
+    if (int st = batch_->status(msg)) throw ScriptError(status_code(st), msg);
     if (thermo_every_ >= 0) emit_thermo(true);
     for (const DumpSpec &d : dumps_)
         if (step_ % d.every == 0) write_dump(d);
@@ -1130,7 +1130,7 @@ void Script::run(long long nsteps)
         check_cuda(cudaStreamSynchronize(batch_->stream()), "run");
         step_ = next;
         if (int st = batch_->status(msg))
-            throw ScriptError(st & kErrNonFinite ? MDPD_ERR_NAN : MDPD_ERR_OVERFLOW, msg);
+            throw ScriptError(status_code(st), msg);
         if (ev_last) emit_thermo(false);
         for (const DumpSpec &d : dumps_)
             if (step_ % d.every == 0) write_dump(d);

@@ -10,9 +10,16 @@
 #include <string>
 #include <vector>
 
+#include "../../include/mdpd.h"
 #include "engine.h"
 
 namespace mdpd {
+
+// the MDPD_* code of a box status word that is not 0
+inline int status_code(int st)
+{
+    return st & kErrTimeout ? MDPD_ERR_TIMEOUT : st & kErrNonFinite ? MDPD_ERR_NAN : MDPD_ERR_OVERFLOW;
+}
 
 class ScriptError : public std::runtime_error {
 public:
