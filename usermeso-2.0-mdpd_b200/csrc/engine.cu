@@ -518,16 +518,18 @@ void Box::download_state(double *x, double *v, double *f, int32_t *tag, int32_t 
 {
     const BoxState st = state();
     const int c = st.cur;
-    std::vector<double> col(n);
-    for (int d = 0; d < 3; ++d) {
-        if (x) {
-            check_cuda(cudaMemcpy(col.data(), desc.x[c][d], sizeof(double) * n, cudaMemcpyDeviceToHost), "download");
-            for (int i = 0; i < n; ++i) x[3 * i + d] = col[i];
-        }
-        if (v) {
-            check_cuda(cudaMemcpy(col.data(), desc.v[c][d], sizeof(double) * n, cudaMemcpyDeviceToHost), "download");
-            for (int i = 0; i < n; ++i) v[3 * i + d] = col[i];
-        }
+    if (x || v) {
+        // interleaved on the device and copied once per array into the caller's memory (component by
+        // component through a host column, x and v of 60,007 particles took 1.03 ms, now 0.69)
+        // scratch: the buffer that is not live, whose x and v (six arrays of n, one after another in the
+        // arena) the next reorder overwrites
+        const size_t n3 = 3 * (size_t)n;
+        double *dx = desc.x[1 - c][0], *dv = dx + n3;
+        launch_gather_rows(0, state_buffers(desc), desc.st, n, x ? dx : nullptr, v ? dv : nullptr);
+        check_cuda(cudaGetLastError(), "download");
+        if (x) check_cuda(cudaMemcpyAsync(x, dx, sizeof(double) * n3, cudaMemcpyDeviceToHost, 0), "download");
+        if (v) check_cuda(cudaMemcpyAsync(v, dv, sizeof(double) * n3, cudaMemcpyDeviceToHost, 0), "download");
+        check_cuda(cudaStreamSynchronize(0), "download");
     }
     if (f) {
         std::vector<float4> ff(n);

@@ -764,6 +764,23 @@ __global__ void k_gather_by_tag(StateBuffers b, const BoxState *__restrict__ st,
     vo[3 * r] = b.v[c][0][i], vo[3 * r + 1] = b.v[c][1][i], vo[3 * r + 2] = b.v[c][2][i];
 }
 
+__global__ void k_gather_rows(StateBuffers b, const BoxState *__restrict__ st, int n, double *__restrict__ xo,
+                              double *__restrict__ vo)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int c = st->cur & 1;
+    for (int d = 0; d < 3; ++d) {
+        if (xo) xo[3 * (size_t)i + d] = b.x[c][d][i];
+        if (vo) vo[3 * (size_t)i + d] = b.v[c][d][i];
+    }
+}
+
+void launch_gather_rows(cudaStream_t s, const StateBuffers &b, const BoxState *st, int n, double *xo, double *vo)
+{
+    if (n > 0 && (xo || vo)) k_gather_rows<<<(n + 255) / 256, 256, 0, s>>>(b, st, n, xo, vo);
+}
+
 void launch_gather_by_tag(cudaStream_t s, const StateBuffers &b, const BoxState *st, int n, double *xo, double *vo)
 {
     if (n > 0) k_gather_by_tag<<<(n + 255) / 256, 256, 0, s>>>(b, st, n, xo, vo);

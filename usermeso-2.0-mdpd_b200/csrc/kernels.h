@@ -92,6 +92,8 @@ struct StateBuffers {
 // x, v of the live buffer (st->cur, read on the device), internal order -> xo[3n], vo[3n] in
 // tag order (tags 1..n)
 void launch_gather_by_tag(cudaStream_t s, const StateBuffers &b, const BoxState *st, int n, double *xo, double *vo);
+// the same in internal order; a null array is skipped
+void launch_gather_rows(cudaStream_t s, const StateBuffers &b, const BoxState *st, int n, double *xo, double *vo);
 void launch_thermo(cudaStream_t s, BoxDesc *boxes, const BatchUnits &u, double *out, int *done);
 void launch_density_profile(cudaStream_t s, const BoxDesc *boxes, int box, const Unit *units,
                             int nunits, int dim, int groupbit, double lo, double inv, int nbin,
