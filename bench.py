@@ -281,8 +281,8 @@ def main():
     r1 = b.rebuild_steps()
     value, t_max = aggregate(ntot * args.steps, ms * args.steps / 1e3, world)
     # a pair-once mDPD step: integrate, density, force (a finalize at the end of the run); a rebuilding
-    # step adds 10 (the scan of the longest boxes takes two kernels)
-    gpu_launches = 3 * args.steps + 1 + 10 * (r1 - r0)
+    # step adds 11 (the scans of the longest boxes take two kernels each)
+    gpu_launches = 3 * args.steps + 1 + 11 * (r1 - r0)
     eq_states = [b.state(k) for k in range(len(cfg))] if not args.no_extras else None
     b.close()
 

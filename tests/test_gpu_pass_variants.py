@@ -208,3 +208,51 @@ def test_one_type_boxes_alone_same_bits_as_in_a_batch():
         assert one.thermo(0).nbuild == two.thermo(1).nbuild and one.rebuild_steps() == two.rebuild_steps()
         one.close()
         two.close()
+
+
+def wall_box(length, wall_rho, exact="fast"):
+    """fluid between frozen walls at the low and high x ends"""
+    L = np.array([length, 5.0, 5.0])
+    rng = np.random.default_rng(4)
+    nf, nw = int(6.05 * (L[0] - 4) * 25), int(wall_rho * 4 * 25)
+    xf = rng.uniform(0, 1, (nf, 3)) * (L - (4, 0, 0)) + (2, 0, 0)
+    xw = rng.uniform(0, 1, (nw, 3)) * (4, 5, 5)
+    xw[:, 0] = np.mod(xw[:, 0] - 2, L[0])
+    v = np.concatenate([rng.normal(0, 1, (nf, 3)), np.zeros((nw, 3))])
+    lam = deck((nf, nw), (0,) * 3, L, "group fluid type 1\ngroup solid type 2",
+               "pair_style mdpd/meso 1.0 1.0 77 fluid solid\npair_coeff * * -10 5 4.5 1.0 0.75\n"
+               f"pair_modify rng {exact}",
+               "fix BC all aboundary/rho/meso cut_rho 0.75 phi_c 0.5 cut_phi 1.0 rho_wall 8.0 wall solid mobile fluid\n"
+               "fix NVE fluid nve/meso", np.concatenate([xf, xw]), v)
+    return lam, L
+
+
+# 17 wall particles per unit volume: near-wall rows hold more than the list of wall particles takes
+# (n_col2), so the wall fix reads those rows whole
+@pytest.mark.parametrize("length,wall_rho", [(12, 8.0), (12, 17.0), (100, 8.0)])
+def test_wall_fraction_from_listed_and_whole_rows(length, wall_rho):
+    a, L = wall_box(length, wall_rho)
+    b, _ = wall_box(length, wall_rho)
+    x0 = a.state()[0]
+    a.setup()
+    b.setup()
+    a.step(6)
+    for _ in range(6):
+        b.step(1)
+    assert same(fields(a, FIELDS + ("phi",)), fields(b, FIELDS + ("phi",)))
+    a.step(1)
+    x, phi, typ = a.field("x"), a.field("phi"), a.field("type")
+    tag = a.field("tag")
+    w = x[typ == 2]
+    assert np.array_equal(w, x0[tag[typ == 2] - 1])  # frozen
+    m = np.nonzero(typ == 1)[0]
+    d = x[m][:, None, :] - w[None]
+    d -= L * np.round(d / L)
+    r = np.sqrt((d * d).sum(2))
+    want = np.where(r < 1, (1 + 3 * r) * np.clip(1 - r, 0, None) ** 3, 0).sum(1) * 105 / (16 * np.pi * 8.0)
+    # a reflected particle (phi above phi_c) has moved since; FP32 coordinates and terms, ~40 of them
+    ok = phi[m] <= 0.5
+    assert ok.sum() > 0.5 * len(m) and (want > 0.01).sum() > 20
+    assert np.abs(phi[m] - want)[ok].max() < 1e-4
+    a.close()
+    b.close()

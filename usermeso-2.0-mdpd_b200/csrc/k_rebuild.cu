@@ -211,8 +211,8 @@ __global__ void __launch_bounds__(256) k_scan(const BoxDesc *__restrict__ boxes,
 static int g_scan_cls[3] = {4, 4, 4}, g_scan_bins[3] = {4, 4, 4};
 
 // In one kernel a block adds up every count before its chunk, which costs less than a second
-// launch (~2.5 us) while a scan has up to kShortScan chunks.
-constexpr int kShortScan = 32;
+// launch (~2.5 us) while a scan has up to kShortScan chunks (29 chunks: 16.7 us, in two kernels 10).
+constexpr int kShortScan = 16;
 
 template <int SELA, int SELB>
 static void scan(cudaStream_t s, BoxDesc *boxes, const UnitList &a, const UnitList &b, int longest, int sms,

@@ -82,6 +82,8 @@ __global__ void __launch_bounds__(kUnit, integrate_blocks(WALL)) k_integrate(Box
             int code8[8];  // image codes of the first ghosts (7 at most unless a side is < 2 cutoffs)
 #pragma unroll
             for (int q = 0; q < 8; ++q) code8[q] = g0 + q < g1 ? B.gimg[g0 + q] : 13;
+            // wall flags are packed on wall-coupled boxes only: without them no row has a wall particle
+            const int nwall = WALL && B.wall_fix && B.arb_bc ? B.count2[i] : 0;
             const double dtfm = B.dtfm[t - 1];
             if (pending) {
                 const int n = B.nlocal;
@@ -110,31 +112,58 @@ __global__ void __launch_bounds__(kUnit, integrate_blocks(WALL)) k_integrate(Box
                 const float cx = (float)x, cy = (float)y, cz = (float)z;
                 double phi_i = 0.0;
                 float nx = 0.f, ny = 0.f, nz = 0.f;
-                const int n = MDPD_IDX(B.count[i], B.n_col + 1);
+                // The row's wall particles as the density pass listed them at the build (most fluid rows
+                // have none); a row that was not listed is read whole.  Four entries at a time, their loads
+                // in flight together.
+                const bool whole = nwall < 0;
+                const int n = whole ? MDPD_IDX(B.count[i], B.n_col + 1) : MDPD_IDX(nwall, B.n_col2 + 1);
+                const int *row2 = B.table2 + (size_t)i * B.n_col2;
                 const float cp = B.cut_phi;
-                for (int k = 0; k < n; ++k) {
-                    const int j = MDPD_IDX(B.table[list_addr(i, k, B.n_col)] & kEntryIndexMask, n_all(B));
-                    const float4 pj = B.pos[j];
-                    if (!(pflags(pj) & 2)) continue;
-                    int s = j, code = 13;
-                    if (j >= B.nlocal) {
-                        s = MDPD_IDX(B.gsrc[j - B.nlocal], B.nlocal);
-                        code = B.gimg[j - B.nlocal];
+                for (int k0 = 0; k0 < n; k0 += 4) {
+                    int j[4], code[4];
+                    double jd[4][3];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int k = k0 + q;
+                        j[q] = -1;
+                        if (k < n)
+                            j[q] = MDPD_IDX((whole ? B.table[list_addr(i, k, B.n_col)] : row2[k]) & kEntryIndexMask,
+                                            n_all(B));
                     }
-                    const float jx = (float)(B.x[c][0][s] + (code % 3 - 1) * B.prd[0]);
-                    const float jy = (float)(B.x[c][1][s] + ((code / 3) % 3 - 1) * B.prd[1]);
-                    const float jz = (float)(B.x[c][2][s] + (code / 9 - 1) * B.prd[2]);
-                    const float dx = cx - jx, dy = cy - jy, dz = cz - jz;
-                    const float rsq = dist2(dx, dy, dz);
-                    if (rsq < cp * cp) {
-                        const float rinv = rsqrtf(rsq);
-                        const float r = fmaxf(rsq * rinv, 1e-10f);
-                        const float d = cp - r;
-                        phi_i += (double)((cp + 3.f * r) * d * d * d * B.phi_factor);
-                        const float w = r * d * d * B.dw_factor * rinv;
-                        nx -= w * dx;
-                        ny -= w * dy;
-                        nz -= w * dz;
+                    if (whole) {
+#pragma unroll
+                        for (int q = 0; q < 4; ++q)
+                            if (j[q] >= 0 && !(pflags(B.pos[j[q]]) & 2)) j[q] = -1;
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        code[q] = 13;
+                        if (j[q] >= B.nlocal) {
+                            code[q] = B.gimg[j[q] - B.nlocal];
+                            j[q] = MDPD_IDX(B.gsrc[j[q] - B.nlocal], B.nlocal);
+                        }
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        for (int d = 0; d < 3; ++d) jd[q][d] = j[q] >= 0 ? B.x[c][d][j[q]] : 0.0;
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        if (j[q] < 0) continue;
+                        const float jx = (float)(jd[q][0] + (code[q] % 3 - 1) * B.prd[0]);
+                        const float jy = (float)(jd[q][1] + ((code[q] / 3) % 3 - 1) * B.prd[1]);
+                        const float jz = (float)(jd[q][2] + (code[q] / 9 - 1) * B.prd[2]);
+                        const float dx = cx - jx, dy = cy - jy, dz = cz - jz;
+                        const float rsq = dist2(dx, dy, dz);
+                        if (rsq < cp * cp) {
+                            const float rinv = rsqrtf(rsq);
+                            const float r = fmaxf(rsq * rinv, 1e-10f);
+                            const float d = cp - r;
+                            phi_i += (double)((cp + 3.f * r) * d * d * d * B.phi_factor);
+                            const float w = r * d * d * B.dw_factor * rinv;
+                            nx -= w * dx;
+                            ny -= w * dy;
+                            nz -= w * dz;
+                        }
                     }
                 }
                 B.phi[c][i] = (float)phi_i;
@@ -328,10 +357,17 @@ void launch_aboundary_meso(cudaStream_t s, BoxDesc *boxes, const BatchUnits &u)
 
 // ---------------------------------------------------------------------------
 // density pass: rho_i = m_i * 15/(2 pi h^5) * sum_{r<h} (h - r)^2 over the list.
-// TPP threads per particle split the list and combine with shuffles.
+// TPP threads per particle split the list and combine with shuffles.  At a build, one thread per
+// particle also lists the row's wall particles (in list order) for the wall fix of the steps after it:
+// the fix then reads ~15 entries of a near-wall row and none of the others instead of all 56 (pore flow,
+// 204,451 particles: integrate pass 167 -> 60 us, step 394 -> 288 us; 511,128: step 830 -> 566 us).
 // ---------------------------------------------------------------------------
+// one thread per particle: 8 gathers in flight in 64 registers (8 blocks per SM) instead of 4 in 32
+constexpr int full_gathers(int tpp) { return tpp == 1 ? 8 : 4; }
+constexpr int full_density_blocks(int tpp) { return tpp == 1 ? 8 : 16 / tpp; }
+
 template <int TPP>
-__global__ void __launch_bounds__(kUnit *TPP, 16 / TPP) k_density(const BoxDesc *__restrict__ boxes,
+__global__ void __launch_bounds__(kUnit *TPP, full_density_blocks(TPP)) k_density(const BoxDesc *__restrict__ boxes,
                                                          const Unit *__restrict__ units, int nunits)
 {
     for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
@@ -343,32 +379,41 @@ __global__ void __launch_bounds__(kUnit *TPP, 16 / TPP) k_density(const BoxDesc 
         const bool live = i < U.end;
         const int c = B.st->cur;
         const bool in_group = live && (B.mask[c][i] & B.rho_bit);
+        const bool list_walls = TPP == 1 && B.wall_fix && B.st->rebuild;
+        int nwall = 0;
+        int *const row2 = B.table2 + (size_t)(live ? i : U.begin) * B.n_col2;
         if (in_group) {
             const float4 pi = B.pos[i];
             const float h = B.cut_rho, h2 = h * h;
             const int n = MDPD_IDX(B.count[i], B.n_col + 1);
             const int ncol = B.n_col;
             const int *row = B.table + ((unsigned)(i & ~31) * (unsigned)ncol + (unsigned)(i & 31));
-            // four independent index -> position gather chains in flight per thread
-            for (int k0 = t; k0 < n; k0 += 4 * TPP) {
-                int j[4];
-                float4 pj[4];
+            // independent index -> position gather chains in flight per thread
+            constexpr int K = full_gathers(TPP);
+            for (int k0 = t; k0 < n; k0 += K * TPP) {
+                int j[K];
+                float4 pj[K];
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
+                for (int q = 0; q < K; ++q) {
                     const int k = k0 + q * TPP;
                     j[q] = k < n ? MDPD_IDX(__ldcs(row + 32 * k) & kEntryIndexMask, n_all(B)) : -1;
                 }
 #pragma unroll
-                for (int q = 0; q < 4; ++q) pj[q] = j[q] >= 0 ? __ldg(&B.pos[j[q]]) : make_float4(1e30f, 0, 0, 0);
+                for (int q = 0; q < K; ++q) pj[q] = j[q] >= 0 ? __ldg(&B.pos[j[q]]) : make_float4(1e30f, 0, 0, 0);
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
+                for (int q = 0; q < K; ++q) {
                     // branchless: (h - r)^2 for 1e-20 <= r^2 < h^2, else 0
                     const float dx = pi.x - pj[q].x, dy = pi.y - pj[q].y, dz = pi.z - pj[q].z;
                     const float rsq = dist2(dx, dy, dz);
                     const float d = (rsq < h2 && rsq >= 1e-20f) ? h - rsq * rsqrtf(rsq) : 0.f;
                     acc = __fmaf_rn(d, d, acc);
+                    if (list_walls && (pflags(pj[q]) & 2)) {
+                        row2[min(nwall, B.n_col2 - 1)] = j[q];
+                        ++nwall;
+                    }
                 }
             }
+            if (list_walls) B.count2[i] = nwall <= B.n_col2 ? nwall : -1;
         }
 #pragma unroll
         for (int o = TPP / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);

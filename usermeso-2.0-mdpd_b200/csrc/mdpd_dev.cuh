@@ -109,7 +109,8 @@ struct BoxDesc {
     // ---- neighbour list (transposed per 32 particles: entry k of i at (i&~31)*n_col + 32k + (i&31)) ----
     int *count, *table;
     // entries within the force cutoff whose source index is above the particle's (each pair
-    // once), compacted by the density pass for the force pass
+    // once), compacted by the density pass for the force pass; on wall-coupled boxes (full-list
+    // passes) the row's wall particles, for the wall fix (count2 -1: not listed, read the whole row)
     int *count2, *table2;
     int n_col2;
     unsigned long long *facc;  // 3 x nlocal fixed-point force sums (2^-32 units), SoA

@@ -246,7 +246,10 @@ __device__ __forceinline__ void permute_particle(const BoxDesc &B, int k, int c,
     B.tag[o][k] = tag;
     B.type[o][k] = type;
     B.mask[o][k] = mask;
-    if (B.wall_fix) B.phi[o][k] = phi;  // zero in both buffers otherwise
+    if (B.wall_fix) {
+        B.phi[o][k] = phi;              // zero in both buffers otherwise
+        if (B.arb_bc) B.count2[k] = -1;  // until the density pass has listed the row's wall particles
+    }
     const float fvx = (float)v[0], fvy = (float)v[1], fvz = (float)v[2];
     B.pos[k] = make_float4((float)(x[0] - B.cen[0]), (float)(x[1] - B.cen[1]),
                            (float)(x[2] - B.cen[2]), pack_w(B, type, mask));
