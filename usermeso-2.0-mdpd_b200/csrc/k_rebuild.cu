@@ -311,7 +311,7 @@ __global__ void __launch_bounds__(kUnit) k_rb_permute(BoxDesc *__restrict__ boxe
 // from the class starts; its packed position goes to bpos as well.  Ghost images take atomic
 // slots after the bin's locals, and the bin sort puts them in index order.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kUnit) k_rb_bins(const BoxDesc *__restrict__ boxes,
+__global__ void __launch_bounds__(kUnit, 7) k_rb_bins(const BoxDesc *__restrict__ boxes,
                                                    const Unit *__restrict__ units, int nunits)
 {
     for (int u = blockIdx.x; u < nunits; u += gridDim.x) {

@@ -33,6 +33,7 @@ struct SmallBar {
     unsigned arrived;
     int abort;
     int moved[3];  // displacement flags of steps k, k + 1, k + 2 (mod 3)
+    int next;      // the list build's next item
 };
 
 struct SmallArgs {
@@ -42,15 +43,16 @@ struct SmallArgs {
     int nsteps, rows, parts, nblocks;
 };
 
-// all blocks of the grid; false when the wait ran out or another block's did
-__device__ __forceinline__ bool grid_barrier(SmallBar *bar, unsigned &target, unsigned nblocks, int *s_flag)
+// all blocks of the grid; false when the wait ran out or another block's did.  s_flag[1]: the word at
+// `also` after the barrier (read by the thread that waits)
+__device__ __forceinline__ bool grid_barrier(SmallBar *bar, unsigned &target, unsigned nblocks, int *s_flag,
+                                             const int *also)
 {
     target += nblocks;
     __syncthreads();
     if (threadIdx.x == 0) {
         int ok = 1;
-        __threadfence();
-        atomicAdd(&bar->arrived, 1u);
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&bar->arrived) : "memory");
         unsigned seen, polls = 0;
         for (;;) {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&bar->arrived) : "memory");
@@ -61,11 +63,11 @@ __device__ __forceinline__ bool grid_barrier(SmallBar *bar, unsigned &target, un
                 break;
             }
         }
-        __threadfence();
-        *s_flag = ok;
+        s_flag[0] = ok;
+        if (also) s_flag[1] = *(const volatile int *)also;
     }
     __syncthreads();
-    return *s_flag != 0;
+    return s_flag[0] != 0;
 }
 
 __device__ __forceinline__ int block_sum(int a, int *s_w)
@@ -172,6 +174,9 @@ __device__ __forceinline__ bool small_integrate(const BoxDesc &B, const SmallSme
     }
     const bool edge = i >= n_bulk;
     const int g0 = edge ? B.gfirst[i] : 0, g1 = edge ? min(B.gfirst[i + 1], B.ghost_cap) : 0;
+    int code[7];  // image codes: 7 ghosts at most (a box side is at least three cutoffs)
+#pragma unroll
+    for (int q = 0; q < 7; ++q) code[q] = g0 + q < g1 ? B.gimg[g0 + q] : 13;
     const uint32_t sg0 = STYLE == 0 ? sig_mdpd(tag, sn) : 0u;
     if (pending) clear_force<STYLE>(B, S, r, i);
     if (m & B.nve_bit) {
@@ -193,7 +198,9 @@ __device__ __forceinline__ bool small_integrate(const BoxDesc &B, const SmallSme
     const float4 vv = make_float4(fvx, fvy, fvz, __uint_as_float(sg));
     B.pos[i] = S.pos[r] = p;
     B.vel[i] = S.vel[r] = vv;
-    for (int g = g0; g < g1; ++g) put_ghost(B, g, B.gimg[g], x[0], x[1], x[2], w, vv);
+#pragma unroll
+    for (int q = 0; q < 7; ++q)
+        if (g0 + q < g1) put_ghost(B, g0 + q, code[q], x[0], x[1], x[2], w, vv);
     return ddx * ddx + ddy * ddy + ddz * ddz > B.triggersq;
 }
 
@@ -297,7 +304,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_run_box(const __grid_const
     extern __shared__ __align__(128) char s_dyn[];
     __shared__ uint32_t s_seed[kSmallMaxSteps + 2];
     __shared__ int s_w[kSmallWarps];
-    __shared__ int s_flag;
+    __shared__ int s_flag[2];
     const BoxDesc &B = A.B;
     const SmallSmem S = small_smem(s_dyn, A.rows);
     constexpr int R = 32 / LPR;                   // rows per warp and round
@@ -313,7 +320,9 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_run_box(const __grid_const
     for (int r = tid; r < nrows; r += kSmallThreads)
         for (int d = 0; d < 6; ++d) S.acc[d][r] = 0u;
     __syncthreads();
-    auto barrier = [&] { return grid_barrier(A.bar, target, (unsigned)A.nblocks, &s_flag); };
+    auto barrier = [&](const int *also = nullptr) {
+        return grid_barrier(A.bar, target, (unsigned)A.nblocks, s_flag, also);
+    };
     bool ok = true;
     for (int k = 0; k < A.nsteps && ok; ++k) {
         const uint32_t sn = s_seed[k + 1];
@@ -323,14 +332,15 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_run_box(const __grid_const
         if (__any_sync(0xffffffffu, moved) && lane == 0) atomicOr(&A.bar->moved[k % 3], 1);
         // the flag after next's slot: last read before this step's first barrier of the step before
         if (blockIdx.x == 0 && tid == 0) A.bar->moved[(k + 1) % 3] = 0;
-        if (!(ok = barrier())) break;
-        const int any = *(volatile int *)&A.bar->moved[k % 3];
+        if (!(ok = barrier(&A.bar->moved[k % 3]))) break;
+        const int any = s_flag[1];
         ++ago;
         rb = 0;
         if (ago >= B.delay && ago % B.every == 0) rb = B.check ? any : 1;
         if (rb) {
             ago = 0;
             ++builds;
+            if (blockIdx.x == 0 && tid == 0) A.bar->next = 0;
             for (int r = tid; r < nrows; r += kSmallThreads) key_particle(B, base + r, cur);
             if (!(ok = barrier())) break;
             {
@@ -374,8 +384,15 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_run_box(const __grid_const
             for (int b0 = 4 * gw; b0 < B.nbin; b0 += 4 * warps)
                 bucket_four<1>(B, b0, B.nbin, reinterpret_cast<unsigned long long *>(S.scratch + w * kSmallScratch));
             if (!(ok = barrier())) break;
-            for (int q = gw; q < B.nbin * A.parts; q += warps)
+            // items from a counter: bins of the shell have no rows and take no time, full ones ~15 us each
+            for (;;) {
+                int q = 0;
+                if (lane == 0) q = atomicAdd(&A.bar->next, 1);
+                q = __shfl_sync(0xffffffffu, q, 0);
+                if (q >= B.nbin * A.parts) break;
                 list_bin(B, q / A.parts, q % A.parts, A.parts, *reinterpret_cast<ListSmem *>(S.scratch + w * kSmallScratch));
+                __syncwarp();
+            }
             if (!(ok = barrier())) break;
         }
         if (STYLE == 0) {
@@ -452,11 +469,11 @@ template <int STYLE> static const void *small_kernel(bool exact, bool uni, int l
     return uni ? small_kernel<STYLE, false, true>(lpr) : small_kernel<STYLE, false, false>(lpr);
 }
 
-// Up to 768 rows per block (113,664 particles on 148 SMs; the force pass gives a warp at most 32
-// rows) the whole run beats a launch per pass, us per step with / without:
-//   mDPD  2,000  25 / 46     8,000  32 / 50    20,000  45 / 57    42,000  52 / 70    70,000  75 / 90
-//       100,000  95 / 107  113,000  99 / 110
-//   DPD   3,000  21 / 50    20,000  27 / 53    56,000  38 / 61    85,000  55 / 74   113,000  65 / 83
+// mDPD up to 768 rows per block (113,664 particles on 148 SMs; the force pass gives a warp at most 32
+// rows), DPD up to 1,400 (what shared memory holds): there the whole run beats a launch per pass, us per
+// step with / without:
+//   mDPD  2,000  23 / 46     8,000  27 / 50    20,000  36 / 57    42,000  48 / 70   100,000  83 / 107
+//   DPD   3,000  19 / 50    20,000  27 / 53    56,000  37 / 61   113,000  61 / 83   200,000 103 / 120
 // Boxes with walls, and the threads-per-particle shapes of the full-list passes other than one, take
 // the launches; so does a box of mostly empty bins, whose bin passes outweigh the rows (a 109,000-particle
 // slab in a box of 30,000 bins: 129 us a step here).
@@ -469,7 +486,7 @@ bool small_run_plan(const BoxDesc &B, const StepConfig &c, SmallPlan &p)
     p.blocks = blocks;
     p.rows = (B.nlocal + blocks - 1) / blocks;
     p.lpr = p.rows <= kSmallWarps ? 32 : p.rows <= 4 * kSmallWarps ? 8 : 2;
-    if (p.rows > 32 * kSmallWarps) return false;
+    if (p.rows > (c.style == 0 ? 32 * kSmallWarps : 1400)) return false;
     const long long inner = (long long)(B.mbin[0] - 2) * (B.mbin[1] - 2) * (B.mbin[2] - 2);
     p.parts = 8;
     while (p.parts > 1 && inner * p.parts > warps) p.parts /= 2;

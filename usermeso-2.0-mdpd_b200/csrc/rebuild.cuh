@@ -189,23 +189,27 @@ __device__ __forceinline__ int image_mask(const BoxDesc &B, double x, int d)
 
 __device__ __forceinline__ int bits_count(int m) { return 1 + (m & 1) + ((m >> 1) & 1); }
 
-// f(sx, sy, sz) for every periodic image of a particle with image masks m, in the order of the
-// ghost indices: z slowest
+// f(q, sx, sy, sz) for the periodic images of a particle with image masks m, in the order of the ghost
+// indices (z slowest), q counting them.  A box side is at least three cutoffs, so a coordinate has
+// one image at most and a particle seven; the eight combinations are unrolled, so that f's loads for
+// all images can be in flight together.
 template <class F> __device__ __forceinline__ void for_images(const int m[3], F &&f)
 {
-    for (int sz = -1; sz <= 1; ++sz) {
-        if (sz == 1 && !(m[2] & 1)) continue;
-        if (sz == -1 && !(m[2] & 2)) continue;
-        for (int sy = -1; sy <= 1; ++sy) {
-            if (sy == 1 && !(m[1] & 1)) continue;
-            if (sy == -1 && !(m[1] & 2)) continue;
-            for (int sx = -1; sx <= 1; ++sx) {
-                if (sx == 1 && !(m[0] & 1)) continue;
-                if (sx == -1 && !(m[0] & 2)) continue;
-                if (sx == 0 && sy == 0 && sz == 0) continue;
-                f(sx, sy, sz);
-            }
+    int q = 0;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        // along each axis the unshifted place comes after a shift by -1 and before one by +1
+        int sh[3];
+        bool ok = true, any = false;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const int up = (c >> d) & 1;
+            const int s = (m[d] & 2) ? (up ? 0 : -1) : up;
+            ok &= m[d] != 0 || !up;
+            any |= s != 0;
+            sh[d] = s;
         }
+        if (ok && any) f(q++, sh[0], sh[1], sh[2]);
     }
 }
 
@@ -269,7 +273,7 @@ __device__ __forceinline__ void permute_particle(const BoxDesc &B, int k, int c,
     B.bin_of[k] = bin;
     warp_add1(B.bin_count, MDPD_IDX(bin, B.nbin));
     if (nimg > 1)
-        for_images(m, [&](int sx, int sy, int sz) {
+        for_images(m, [&](int, int sx, int sy, int sz) {
             atomicAdd(&B.bin_count[MDPD_IDX(image_bin(B, x, sx, sy, sz), B.nbin)], 1);
         });
 }
@@ -305,8 +309,24 @@ __device__ __forceinline__ void bins_particle(const BoxDesc &B, int k, int c, in
         m[d] = image_mask(B, x[d], d);
     }
     const float4 vk = B.vel[k];
-    int g = g0;
-    for_images(m, [&](int sx, int sy, int sz) {
+    // the images' bins and the number of locals in them first: their loads are in flight together
+    int gb[7], nloc[7];
+#pragma unroll
+    for (int q = 0; q < 7; ++q) gb[q] = -1, nloc[q] = 0;
+    for_images(m, [&](int q, int sx, int sy, int sz) {
+        const int bn = MDPD_IDX(image_bin(B, x, sx, sy, sz), B.nbin);
+#pragma unroll
+        for (int e = 0; e < 7; ++e)
+            if (e == q) gb[e] = bn;
+    });
+#pragma unroll
+    for (int q = 0; q < 7; ++q)
+        if (gb[q] >= 0) nloc[q] = bin_locals(B, gb[q]);
+#pragma unroll
+    for (int q = 0; q < 7; ++q)
+        if (gb[q] >= 0 && g0 + q < B.ghost_cap) nloc[q] += atomicAdd(&B.bin_cursor[gb[q]], 1);
+    for_images(m, [&](int q, int sx, int sy, int sz) {
+        const int g = g0 + q;
         if (g >= B.ghost_cap) {
             atomicOr(&B.st->status, kErrGhostOverflow);
             return;
@@ -318,10 +338,12 @@ __device__ __forceinline__ void bins_particle(const BoxDesc &B, int k, int c, in
         B.pos[gi] = make_float4((float)(x[0] + sx * B.prd[0] - B.cen[0]), (float)(x[1] + sy * B.prd[1] - B.cen[1]),
                                 (float)(x[2] + sz * B.prd[2] - B.cen[2]), ghost_w(pk.w, code));
         B.vel[gi] = vk;
-        const int gb = MDPD_IDX(image_bin(B, x, sx, sy, sz), B.nbin);
-        const int q = MDPD_IDX(bin_locals(B, gb) + atomicAdd(&B.bin_cursor[gb], 1), na);
-        if (q < na) B.bin_order[q] = gi;
-        ++g;
+#pragma unroll
+        for (int e = 0; e < 7; ++e)
+            if (e == q) {
+                const int at = MDPD_IDX(nloc[e], na);
+                if (at < na) B.bin_order[at] = gi;
+            }
     });
 }
 
@@ -349,15 +371,15 @@ struct ListSmem {
     int d[32], ex[32];          // non-empty stencil bins: start - stream offset; offset
 };
 
-// rows of bin b by one warp; with parts > 1 the bin's centres are taken `per` at a time by `parts`
-// warps (32 / parts each)
+// rows of bin b by one warp; with parts > 1 the bin's members are shared out to `parts` warps
 __device__ __forceinline__ void list_bin(const BoxDesc &B, int b, int part, int parts, ListSmem &L)
 {
-    const int lane = threadIdx.x & 31, per = 32 / parts;
+    const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
     const int s = B.bin_start[b], e = B.bin_start[b + 1];
     if (e == s) return;
     if (!(MDPD_IN(s, e) && MDPD_IN(e - 1, n_all(B)))) return;  // check build: a bin outside the arrays
+    const int per = parts == 1 ? 32 : min(32, (e - s + parts - 1) / parts);  // centres at a time
     if (B.bin_order[s] >= B.nlocal) return;  // no locals in this bin
     const float rc2 = B.rc2_tail;
     const float rn2 = B.list_reduce ? B.rn2_list : rc2;  // with rc2: every pair (full list)
