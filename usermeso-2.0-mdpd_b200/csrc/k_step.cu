@@ -448,11 +448,16 @@ void launch_density(cudaStream_t s, BoxDesc *boxes, const BatchUnits &u, const S
 // two signatures.  Epilogue (t==0): store f, final half-kick (FP64 v, body force in FP64).
 // ---------------------------------------------------------------------------
 constexpr int kQueue = 16;  // list entries tested per phase-1 round of the force pass
+constexpr int kTests = 4;   // of them with their gathers in flight together
 
-// 8 blocks of 128 threads per SM (64 registers): measured faster on a wall-coupled box than 10
-// blocks at 48 registers, which spilled
+// Blocks of 128 threads per SM at one thread per particle.  The pass waits on its gathers (6 cycles of
+// long-scoreboard stall per issued instruction, L1 53 %, issue 57 %).  Classic DPD, 1M particles: 8 blocks
+// (64 registers) 185 us, 7 blocks 204, 6 blocks 200; without the next pair's loads ahead 193.
+// Wall-coupled mDPD, step of 204,451 particles: 8 blocks 289 us, 7 blocks 281, 6 blocks (80 registers) 277.
+constexpr int full_force_blocks(bool wallc) { return wallc ? 6 : 8; }
+
 template <int TPP, int STYLE, bool EXACT, bool EV, bool WALLC, bool UNI>
-__global__ void __launch_bounds__(kUnit *TPP, 8 / TPP) k_force(const BoxDesc *__restrict__ boxes,
+__global__ void __launch_bounds__(kUnit *TPP, TPP == 1 ? full_force_blocks(WALLC) : 8 / TPP) k_force(const BoxDesc *__restrict__ boxes,
                                                        const Unit *__restrict__ units, int nunits, int kick)
 {
     __shared__ PairCoeff s_coeff[kMaxTypes * kMaxTypes];
@@ -503,19 +508,19 @@ __global__ void __launch_bounds__(kUnit *TPP, 8 / TPP) k_force(const BoxDesc *__
                 // in-range neighbours are queued (this thread's column of s_q)
                 int nq = 0;
 #pragma unroll
-                for (int b4 = 0; b4 < kQueue; b4 += 4) {
-                    int j[4];
-                    float4 pj[4];
+                for (int b4 = 0; b4 < kQueue; b4 += kTests) {
+                    int j[kTests];
+                    float4 pj[kTests];
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
+                    for (int q = 0; q < kTests; ++q) {
                         const int k = kb + (b4 + q) * TPP;
                         j[q] = k < n ? MDPD_IDX(__ldcs(row + 32 * k) & kEntryIndexMask, n_all(B)) : -1;
                     }
 #pragma unroll
-                    for (int q = 0; q < 4; ++q)
+                    for (int q = 0; q < kTests; ++q)
                         pj[q] = j[q] >= 0 ? __ldg(&B.pos[j[q]]) : make_float4(1e30f, 0, 0, 0);
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
+                    for (int q = 0; q < kTests; ++q) {
                         const float dx = pi.x - pj[q].x, dy = pi.y - pj[q].y, dz = pi.z - pj[q].z;
                         const float rsq = dist2(dx, dy, dz);
                         const int cid = UNI ? 0 : ti * ntype + ptype(pj[q]);
@@ -523,12 +528,26 @@ __global__ void __launch_bounds__(kUnit *TPP, 8 / TPP) k_force(const BoxDesc *__
                             s_q[nq++][threadIdx.x] = j[q];
                     }
                 }
-                // phase 2: forces of the queued neighbours, in list order
-                for (int q = 0; q < nq; ++q) {
+                // phase 2: forces of the queued neighbours, in list order; the next one's position,
+                // velocity and density are loaded while the current pair is evaluated
+                float4 pjn, vjn;
+                float rjn = 0.f;
+                auto load = [&](int q) {
                     const int j = s_q[q][threadIdx.x];
-                    const float4 pj = __ldg(&B.pos[j]);
-                    pair_term<STYLE, EXACT, EV, WALLC>(B, s_coeff[UNI ? 0 : ti * ntype + ptype(pj)], j, pj, pi, vi, si,
-                                                       rho_i, i_mobile, wall_ratio, wall_sqrt, dtis, fx, fy, fz, ev);
+                    pjn = __ldg(&B.pos[j]);
+                    vjn = __ldg(&B.vel[j]);
+                    if (STYLE == 0) rjn = __ldg(&B.rho[j]);
+                };
+                if (nq > 0) load(0);
+                for (int q = 0; q < nq; ++q) {
+                    const float4 pj = pjn, vj = vjn;
+                    const float rho_j = rjn;
+                    if (q + 1 < nq) load(q + 1);
+                    const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+                    pair_core<STYLE, EXACT, EV, WALLC>(s_coeff[UNI ? 0 : ti * ntype + ptype(pj)], dx, dy, dz,
+                                                       dist2(dx, dy, dz), vi, vj, si, rho_i, rho_j,
+                                                       WALLC && i_mobile && (pflags(pj) & 2), wall_ratio, wall_sqrt, dtis,
+                                                       fx, fy, fz, ev);
                 }
             }
         }

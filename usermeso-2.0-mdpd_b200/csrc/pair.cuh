@@ -75,22 +75,4 @@ __device__ __forceinline__ void pair_core(const PairCoeff &cf, float dx, float d
     }
 }
 
-// one pair's contribution to particle i, loading j's velocity and density only when the pair
-// is inside the type-pair cutoff
-template <int STYLE, bool EXACT, bool EV, bool WALLC>
-__device__ __forceinline__ void pair_term(const BoxDesc &B, const PairCoeff &cf, int j, const float4 &pj,
-                                          const float4 &pi, const float4 &vi, uint32_t si, float rho_i,
-                                          bool i_mobile, float wall_ratio, float wall_sqrt, float dtis, float &fx,
-                                          float &fy, float &fz, EvAcc &ev)
-{
-    const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
-    const float rsq = dist2(dx, dy, dz);
-    if (!(rsq < cf.cutsq && rsq >= 1e-20f)) return;
-    const float4 vj = __ldg(&B.vel[j]);
-    const float rho_j = STYLE == 0 ? __ldg(&B.rho[j]) : 0.f;
-    pair_core<STYLE, EXACT, EV, WALLC>(cf, dx, dy, dz, rsq, vi, vj, si, rho_i, rho_j,
-                                       WALLC && i_mobile && (pflags(pj) & 2), wall_ratio, wall_sqrt, dtis, fx, fy,
-                                       fz, ev);
-}
-
 }  // namespace mdpd
