@@ -475,13 +475,13 @@ template <int STYLE> static const void *small_kernel(bool exact, bool uni, int l
 //   mDPD  2,000  23 / 46     8,000  27 / 50    20,000  36 / 57    42,000  48 / 70   100,000  83 / 107
 //   DPD   3,000  19 / 50    20,000  27 / 53    56,000  37 / 61   113,000  61 / 83   200,000 103 / 120
 // Boxes with walls, and the threads-per-particle shapes of the full-list passes other than one, take
-// the launches; so does a box of mostly empty bins, whose bin passes outweigh the rows (a 109,000-particle
-// slab in a box of 30,000 bins: 129 us a step here).
+// the launches.  Mostly empty bins cost either way; up to a bin per particle the run is still ahead (slabs:
+// 109,000 particles, 30,000 bins 107 / 132; 24,200 particles, 9,200 bins 53 / 82).
 bool small_run_plan(const BoxDesc &B, const StepConfig &c, SmallPlan &p)
 {
     if (c.full_chip || c.wall || c.wall_coupling || c.aboundary) return false;
     if (c.style == 0 ? !c.half : c.tpp_force != 1) return false;
-    if (B.nbin > B.nlocal / 5 + 4096) return false;  // uniform fluids: a bin per 6 to 13 particles
+    if (B.nbin > B.nlocal + 4096) return false;  // uniform fluids: a bin per 6 to 13 particles
     const int blocks = c.sms, warps = blocks * kSmallWarps;
     p.blocks = blocks;
     p.rows = (B.nlocal + blocks - 1) / blocks;
