@@ -175,7 +175,8 @@ int mdpd_batch_run_thermo(mdpd_batch_t *b, int64_t nsteps, mdpd_thermo_t *out, i
  * warp shares its 32 particles' pairs out to its 32 lanes, its compact rows staged in shared
  * memory first) or 0 (the same shares, each entry read from the table in the pair loop).
  * Full-list batches (classic DPD, wall-coupled mDPD): threads per particle of the density and
- * force passes (1, 2 or 4 each). */
+ * force passes (1, 2 or 4 each); a single small box, whose runs go in one launch with one thread per
+ * particle, keeps 1 and 1. */
 int mdpd_batch_tune(mdpd_batch_t *b, int32_t *shape_density, int32_t *shape_force);
 /* mdpd_batch_tune with its picks persisted in a JSON file (path; created when absent):
  * {"version": 1, "entries": {"<key>": {"density": D, "force": F, "ms_per_step": T}}} (T: the pick's pair

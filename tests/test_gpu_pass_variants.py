@@ -256,3 +256,15 @@ def test_wall_fraction_from_listed_and_whole_rows(length, wall_rho):
     assert np.abs(phi[m] - want)[ok].max() < 1e-4
     a.close()
     b.close()
+
+
+def test_tuner_keeps_the_one_launch_runs_of_a_small_box():
+    b = mdpd.Batch([mdpd.box_spec(3000, 10.0, style=1, A=25.0, rho_est=0.0, seed=5, init_seed=6)])
+    b.setup()
+    b.step(5)
+    x, v = b.state(0)
+    assert b.tune() == (1, 1)
+    assert np.array_equal(b.state(0)[0], x) and b.thermo(0).step == 5
+    b.step(5)
+    assert b.thermo(0).status == 0
+    b.close()

@@ -155,6 +155,8 @@ public:
     // copies queued on the batch's stream through one scratch of the largest box, one wait
     void download_all(double *const *x, double *const *v);
     cudaStream_t stream() const { return stream_; }
+    // whether runs of plain steps go in one cooperative launch (k_small.cu) with the present shapes
+    bool whole_runs() const { return small_.kernel != nullptr; }
     const std::vector<Box *> &boxes() const { return boxes_; }
     StepConfig cfg;
     BatchUnits units;
