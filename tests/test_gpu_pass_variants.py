@@ -1,5 +1,7 @@
 """Launch shapes that depend on the size of the work: every shape gives the same bits, and the
 smallest one agrees with the FP64 oracle engine."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -268,3 +270,34 @@ def test_tuner_keeps_the_one_launch_runs_of_a_small_box():
     b.step(5)
     assert b.thermo(0).status == 0
     b.close()
+
+
+def test_small_boxes_stepped_by_several_threads():
+    """runs of different boxes from several host threads: each as it is alone"""
+    def make(k):
+        n = 2500 + 700 * k
+        kw = dict(style=1, A=25.0, rho_est=0.0) if k % 2 else {}
+        return mdpd.Batch([mdpd.box_spec(n, (n / (3.0 if k % 2 else RHO)) ** (1 / 3), seed=k + 1, init_seed=k + 7, **kw)])
+
+    def go(k, out):
+        try:
+            b = make(k)
+            b.setup()
+            for _ in range(6):
+                b.step(60)
+            out[k] = b.state(0)
+            b.close()
+        except Exception as e:  # seen by the main thread
+            out[k] = e
+
+    alone, together = {}, {}
+    for k in range(4):
+        go(k, alone)
+    th = [threading.Thread(target=go, args=(k, together)) for k in range(4)]
+    for t in th:
+        t.start()
+    for t in th:
+        t.join()
+    for k in range(4):
+        assert not isinstance(together[k], Exception), together[k]
+        assert same(alone[k], together[k])

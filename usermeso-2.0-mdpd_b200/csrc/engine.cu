@@ -772,12 +772,32 @@ void Batch::plan_small()
     if (small_.kernel && !d_bar_) d_bar_ = batch_alloc<char>(small_bar_bytes(), stream_);
 }
 
+// A small box's run needs a block on every SM at once.  Runs of several streams and threads therefore
+// follow one another on the device: each waits for the end of the one launched before it (two could not
+// be resident together anyway), so no run can hold SMs that another one's unplaced blocks wait for.
+static cudaError_t ordered_small_run(cudaStream_t s, const BoxDesc &B, const SmallPlan &p, void *bar, int *done,
+                                     long long nsteps)
+{
+    static std::mutex mu;
+    static cudaEvent_t last[64] = {};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+    std::lock_guard<std::mutex> lock(mu);
+    if (!last[dev] && (e = cudaEventCreateWithFlags(&last[dev], cudaEventDisableTiming)) != cudaSuccess) return e;
+    if ((e = cudaStreamWaitEvent(s, last[dev], 0)) != cudaSuccess) return e;
+    const cudaError_t run = launch_small_run(s, B, p, bar, done, nsteps);
+    e = cudaEventRecord(last[dev], s);
+    return run != cudaSuccess ? run : e;
+}
+
 void Batch::run(long long nsteps, bool sync, bool ev_last)
 {
     Range r("mdpd::run");
     const long long plain = nsteps - (ev_last && nsteps > 0 ? 1 : 0);
-    if (small_.kernel) {
-        const cudaError_t e = launch_small_run(stream_, one_, small_, d_bar_, d_done, plain);
+    if (small_.kernel && plain > 0) {
+        const cudaError_t e = ordered_small_run(stream_, one_, small_, d_bar_, d_done, plain);
         if (e == cudaErrorCooperativeLaunchTooLarge) {  // part of the device is taken (MPS): nothing was launched
             (void)cudaGetLastError();
             small_.kernel = nullptr;
