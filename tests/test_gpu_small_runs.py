@@ -1,0 +1,66 @@
+"""Runs of small boxes in one launch: several boxes, threads and refused launches side by side."""
+import threading
+
+import numpy as np
+import pytest
+
+import mdpd
+
+pytestmark = pytest.mark.gpu
+
+DPD = dict(style=1, A=25.0, rho_est=0.0)
+
+
+def batch(n, style=0, seed=1, exact=0):
+    kw = dict(DPD) if style else {}
+    return mdpd.Batch([mdpd.box_spec(n, (n / (3.0 if style else 6.05)) ** (1 / 3), seed=seed, init_seed=seed + 6,
+                                     exact_rng=exact, **kw)])
+
+
+def same(a, b):
+    return all(np.array_equal(p, q) for p, q in zip(a, b))
+
+
+# pairs of sizes whose runs share a kernel (32, 8 and 2 lanes per row on 148 SMs: up to 24, up to 96 and
+# more rows per block) but not the amount of shared memory
+@pytest.mark.parametrize("large,small", [(3000, 2000), (9000, 5000), (20000, 15000)])
+@pytest.mark.parametrize("style", [0, 1])
+def test_boxes_that_share_a_run_kernel(style, large, small):
+    """the larger box's batch is made first, then the smaller one's; both step on in turn, then from a
+    thread each: every box as it is alone"""
+    sizes = (large, small)
+
+    def alone(k):
+        b = batch(sizes[k], style, seed=k + 1)
+        b.setup()
+        for _ in range(6):
+            b.step(7)
+        s = b.state(0)
+        b.close()
+        return s
+
+    want = [alone(k) for k in range(2)]
+    bs = [batch(sizes[k], style, seed=k + 1) for k in range(2)]
+    for b in bs:
+        b.setup()
+    for _ in range(3):
+        for b in bs:
+            b.step(7)
+    errors = []
+
+    def go(b):
+        try:
+            for _ in range(3):
+                b.step(7)
+        except Exception as e:  # seen by the main thread
+            errors.append(e)
+
+    th = [threading.Thread(target=go, args=(b,)) for b in bs]
+    for t in th:
+        t.start()
+    for t in th:
+        t.join()
+    assert not errors, errors
+    for k in range(2):
+        assert same(bs[k].state(0), want[k])
+        bs[k].close()

@@ -798,8 +798,8 @@ void Batch::run(long long nsteps, bool sync, bool ev_last)
     const long long plain = nsteps - (ev_last && nsteps > 0 ? 1 : 0);
     if (small_.kernel && plain > 0) {
         const cudaError_t e = ordered_small_run(stream_, one_, small_, d_bar_, d_done, plain);
+        if (e != cudaSuccess) (void)cudaGetLastError();  // a refused launch is not left for the next caller
         if (e == cudaErrorCooperativeLaunchTooLarge) {  // part of the device is taken (MPS): nothing was launched
-            (void)cudaGetLastError();
             small_.kernel = nullptr;
             capture(0);
         } else {

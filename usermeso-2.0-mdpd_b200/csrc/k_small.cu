@@ -493,11 +493,17 @@ bool small_run_plan(const BoxDesc &B, const StepConfig &c, SmallPlan &p)
     p.smem = small_row_bytes(p.rows) + kSmallWarps * kSmallScratch;
     p.kernel = c.style == 0 ? small_kernel<0>(c.exact_rng, c.uniform_types, p.lpr)
                             : small_kernel<1>(c.exact_rng, c.uniform_types, p.lpr);
-    // one block per SM has to be resident at once: the barriers count on it
-    int per_sm = 0, dev = 0, coop = 0;
+    // One block per SM has to be resident at once: the barriers count on it.  The kernel's limit of dynamic
+    // shared memory belongs to the kernel, which boxes of other sizes share: it is set to what the device
+    // offers, the same value for every box, so that no box's plan lowers another's.
+    int per_sm = 0, dev = 0, coop = 0, optin = 0;
+    cudaFuncAttributes fa;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
-        cudaFuncSetAttribute(p.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, p.smem) != cudaSuccess ||
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+        cudaFuncGetAttributes(&fa, p.kernel) != cudaSuccess || p.smem > optin - (int)fa.sharedSizeBytes ||
+        cudaFuncSetAttribute(p.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             optin - (int)fa.sharedSizeBytes) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, p.kernel, kSmallThreads, p.smem) != cudaSuccess ||
         per_sm < 1) {
         (void)cudaGetLastError();
