@@ -194,6 +194,11 @@ int mdpd_batch_tune_cached(mdpd_batch_t *b, const char *path, int32_t *shape_den
  * the batch's pass family offers, else MDPD_ERR_ARG.  No reference counterpart: the reference's
  * launch shapes come from its occupancy table (occupancy_meso.cu:8-50). */
 int mdpd_batch_set_shapes(mdpd_batch_t *b, int32_t shape_density, int32_t shape_force);
+/* for tests: the batch's one-launch runs poll at most `polls` times at each of their grid barriers
+ * (rounded up to 1024; 0: the default, about 2 s), and from barrier number `barrier` of a launch on
+ * (from 1; 0: none) wait for an arrival that does not come.  Such a run ends with MDPD_ERR_TIMEOUT; its
+ * box stays so: every later call that steps it or sets it up returns MDPD_ERR_TIMEOUT. */
+int mdpd_batch_test_run_wait(mdpd_batch_t *b, uint32_t polls, uint32_t barrier);
 /* last per-step device time in milliseconds measured with CUDA events over nsteps */
 int mdpd_batch_time(mdpd_batch_t *b, int64_t nsteps, double *ms_per_step);
 /* nsteps un-captured steps with CUDA events around each kernel group (same kernels as the

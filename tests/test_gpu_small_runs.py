@@ -64,3 +64,44 @@ def test_boxes_that_share_a_run_kernel(style, large, small):
     for k in range(2):
         assert same(bs[k].state(0), want[k])
         bs[k].close()
+
+
+# barriers of a step that rebuilds: 1 after integrate, 2 to 10 between and after the rebuild's passes (2: the
+# classes are counted, their counts not yet cleared), 11 after the density pass (mDPD), then the force pass's
+@pytest.mark.parametrize("style,barrier", [(0, k) for k in range(1, 13)] + [(1, k) for k in (1, 2, 5, 10, 11)])
+def test_a_barrier_wait_that_runs_out(style, barrier):
+    """one arrival too few with a limit of a few ms: the call says so, whatever was queued behind it is
+    skipped or stays in bounds, the box stays refused, and other boxes step on"""
+    n = 2000
+    kw = dict(DPD) if style else {}
+    L = (n / (3.0 if style else 6.05)) ** (1 / 3)
+    spec = mdpd.box_spec(n, L, check=0, seed=3, init_seed=4, **kw)  # a rebuild at every step
+    other = batch(2500, style)
+    other.setup()
+    ref = batch(2500, style)
+    ref.setup()
+    b = mdpd.Batch([spec])
+    b.setup()
+    b.step(3)
+
+    def refused(f):
+        with pytest.raises(mdpd.MdpdError) as e:
+            f()
+        assert e.value.code == mdpd.ERR_TIMEOUT and "wait" in str(e.value)
+
+    assert mdpd.lib().mdpd_batch_test_run_wait(b.h, 8192, barrier) == mdpd.OK
+    refused(lambda: b.step(600))
+    assert mdpd.lib().mdpd_batch_test_run_wait(b.h, 0, 0) == mdpd.OK
+    other.step(20)
+    refused(lambda: b.step(3))
+    refused(lambda: b.run_thermo(2))
+    refused(lambda: b.time(2))
+    refused(lambda: b.setup())
+    assert b.thermo(0).status & 128
+    b.close()
+    other.step(20)
+    ref.step(20)
+    ref.step(20)
+    assert same(other.state(0), ref.state(0))
+    other.close()
+    ref.close()

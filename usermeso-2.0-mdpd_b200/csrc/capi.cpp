@@ -722,6 +722,16 @@ int mdpd_batch_set_shapes(mdpd_batch_t *b, int32_t shape_density, int32_t shape_
     });
 }
 
+int mdpd_batch_test_run_wait(mdpd_batch_t *b, uint32_t polls, uint32_t barrier)
+{
+    if (!b) return MDPD_ERR_ARG;
+    SmallWait w;
+    if (polls) w.polls = polls;
+    w.barrier = barrier;
+    b->batch->set_run_wait(w);
+    return MDPD_OK;
+}
+
 int mdpd_jobs_validate(const char *spec_path, int32_t *njobs, uint64_t *bytes)
 {
     if (!spec_path) return MDPD_ERR_ARG;

@@ -721,8 +721,9 @@ __global__ void k_set_rebuild(BoxDesc *boxes, const int *which, int nwhich, int 
     for (int b = threadIdx.x; b < nbox; b += blockDim.x) boxes[b].st->rebuild = 0;
     __syncthreads();
     for (int k = threadIdx.x; k < nwhich; k += blockDim.x) {
-        boxes[which[k]].st->rebuild = 1;
-        boxes[which[k]].st->ago = 0;
+        BoxState &S = *boxes[which[k]].st;
+        S.rebuild = !(S.status & kErrTimeout);
+        S.ago = 0;
     }
 }
 
@@ -775,8 +776,8 @@ void Batch::plan_small()
 // A small box's run needs a block on every SM at once.  Runs of several streams and threads therefore
 // follow one another on the device: each waits for the end of the one launched before it (two could not
 // be resident together anyway), so no run can hold SMs that another one's unplaced blocks wait for.
-static cudaError_t ordered_small_run(cudaStream_t s, const BoxDesc &B, const SmallPlan &p, void *bar, int *done,
-                                     long long nsteps)
+static cudaError_t ordered_small_run(cudaStream_t s, const BoxDesc &B, const SmallPlan &p, const SmallWait &w,
+                                     void *bar, int *done, long long nsteps)
 {
     static std::mutex mu;
     static cudaEvent_t last[64] = {};
@@ -787,7 +788,7 @@ static cudaError_t ordered_small_run(cudaStream_t s, const BoxDesc &B, const Sma
     std::lock_guard<std::mutex> lock(mu);
     if (!last[dev] && (e = cudaEventCreateWithFlags(&last[dev], cudaEventDisableTiming)) != cudaSuccess) return e;
     if ((e = cudaStreamWaitEvent(s, last[dev], 0)) != cudaSuccess) return e;
-    const cudaError_t run = launch_small_run(s, B, p, bar, done, nsteps);
+    const cudaError_t run = launch_small_run(s, B, p, w, bar, done, nsteps);
     e = cudaEventRecord(last[dev], s);
     return run != cudaSuccess ? run : e;
 }
@@ -797,7 +798,7 @@ void Batch::run(long long nsteps, bool sync, bool ev_last)
     Range r("mdpd::run");
     const long long plain = nsteps - (ev_last && nsteps > 0 ? 1 : 0);
     if (small_.kernel && plain > 0) {
-        const cudaError_t e = ordered_small_run(stream_, one_, small_, d_bar_, d_done, plain);
+        const cudaError_t e = ordered_small_run(stream_, one_, small_, wait_, d_bar_, d_done, plain);
         if (e != cudaSuccess) (void)cudaGetLastError();  // a refused launch is not left for the next caller
         if (e == cudaErrorCooperativeLaunchTooLarge) {  // part of the device is taken (MPS): nothing was launched
             small_.kernel = nullptr;

@@ -157,6 +157,7 @@ public:
     cudaStream_t stream() const { return stream_; }
     // whether runs of plain steps go in one cooperative launch (k_small.cu) with the present shapes
     bool whole_runs() const { return small_.kernel != nullptr; }
+    void set_run_wait(const SmallWait &w) { wait_ = w; }  // tests
     const std::vector<Box *> &boxes() const { return boxes_; }
     StepConfig cfg;
     BatchUnits units;
@@ -168,6 +169,7 @@ private:
     int *d_done = nullptr;
     BoxDesc one_;                  // a single box's descriptor as the passes see it
     SmallPlan small_;              // its whole-run launch (kernel: null when the box takes the graphs)
+    SmallWait wait_;
     char *d_bar_ = nullptr;
     double *d_thermo = nullptr;
     BoxState *d_states = nullptr;  // gathered copies of the boxes' scalars

@@ -16,7 +16,9 @@
 // shared memory between its passes.
 //
 // Every barrier wait is bounded: a block that waits too long raises the run's abort flag, and every
-// block leaves the kernel with the box's kErrTimeout status set.
+// block that finds it leaves the kernel and sets the box's kErrTimeout status.  The box may then be
+// between two passes (bucket counts of half a rebuild): later runs return at once, and the other passes
+// do not rebuild such a box (its lists of the last build stay in bounds).
 #include "kernels.h"
 #include "pair_rows.cuh"
 #include "rebuild.cuh"
@@ -27,7 +29,6 @@ namespace mdpd {
 
 constexpr int kSmallWarps = 24, kSmallThreads = 32 * kSmallWarps;
 constexpr int kSmallMaxSteps = 256;           // steps per launch (their seeds are formed up front)
-constexpr unsigned kBarrierPolls = 1u << 22;  // ~2 s
 
 struct SmallBar {
     unsigned arrived;
@@ -41,23 +42,26 @@ struct SmallArgs {
     SmallBar *bar;
     int *done;
     int nsteps, rows, parts, nblocks;
+    unsigned polls;     // of a barrier wait, at most
+    unsigned withhold;  // the barrier target from which on one arrival more is waited for (tests)
 };
 
 // all blocks of the grid; false when the wait ran out or another block's did.  s_flag[1]: the word at
 // `also` after the barrier (read by the thread that waits)
-__device__ __forceinline__ bool grid_barrier(SmallBar *bar, unsigned &target, unsigned nblocks, int *s_flag,
-                                             const int *also)
+__device__ __forceinline__ bool grid_barrier(const SmallArgs &A, unsigned &target, int *s_flag, const int *also)
 {
-    target += nblocks;
+    SmallBar *const bar = A.bar;
+    target += (unsigned)A.nblocks;
     __syncthreads();
     if (threadIdx.x == 0) {
         int ok = 1;
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&bar->arrived) : "memory");
+        const unsigned want = target + (target >= A.withhold ? 1u : 0u);
         unsigned seen, polls = 0;
         for (;;) {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&bar->arrived) : "memory");
-            if ((int)(seen - target) >= 0) break;
-            if ((++polls & 1023u) == 0 && (polls >= kBarrierPolls || *(volatile int *)&bar->abort)) {
+            if ((int)(seen - want) >= 0) break;
+            if ((++polls & 1023u) == 0 && (polls >= A.polls || *(volatile int *)&bar->abort)) {
                 *(volatile int *)&bar->abort = 1;
                 ok = 0;
                 break;
@@ -319,11 +323,10 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_run_box(const __grid_const
     for (int k = tid; k < A.nsteps + 2; k += kSmallThreads) s_seed[k] = seed_now(B.seed, S0.step + k);
     for (int r = tid; r < nrows; r += kSmallThreads)
         for (int d = 0; d < 6; ++d) S.acc[d][r] = 0u;
+    if (tid == 0) s_flag[0] = !(S0.status & kErrTimeout);  // an earlier run gave up: nothing is done
     __syncthreads();
-    auto barrier = [&](const int *also = nullptr) {
-        return grid_barrier(A.bar, target, (unsigned)A.nblocks, s_flag, also);
-    };
-    bool ok = true;
+    auto barrier = [&](const int *also = nullptr) { return grid_barrier(A, target, s_flag, also); };
+    bool ok = s_flag[0] != 0;
     for (int k = 0; k < A.nsteps && ok; ++k) {
         const uint32_t sn = s_seed[k + 1];
         bool moved = false;
@@ -417,7 +420,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_run_box(const __grid_const
         ok = barrier();
     }
     if (!ok) {
-        if (tid == 0 && blockIdx.x == 0) atomicOr(&B.st->status, kErrTimeout);
+        if (tid == 0) atomicOr(&B.st->status, kErrTimeout);
         return;
     }
     // the last step's final half-kick
@@ -514,7 +517,8 @@ bool small_run_plan(const BoxDesc &B, const StepConfig &c, SmallPlan &p)
 
 size_t small_bar_bytes() { return sizeof(SmallBar); }
 
-cudaError_t launch_small_run(cudaStream_t s, const BoxDesc &B, const SmallPlan &p, void *bar, int *done, long long nsteps)
+cudaError_t launch_small_run(cudaStream_t s, const BoxDesc &B, const SmallPlan &p, const SmallWait &w, void *bar,
+                             int *done, long long nsteps)
 {
     SmallArgs a;
     a.B = B;
@@ -523,6 +527,8 @@ cudaError_t launch_small_run(cudaStream_t s, const BoxDesc &B, const SmallPlan &
     a.rows = p.rows;
     a.parts = p.parts;
     a.nblocks = p.blocks;
+    a.polls = w.polls;
+    a.withhold = w.barrier ? w.barrier * (unsigned)p.blocks : 0xffffffffu;
     while (nsteps > 0) {
         a.nsteps = (int)std::min<long long>(nsteps, kSmallMaxSteps);
         cudaError_t e = cudaMemsetAsync(bar, 0, sizeof(SmallBar), s);

@@ -229,6 +229,7 @@ __global__ void __launch_bounds__(kUnit, integrate_blocks(WALL)) k_integrate(Box
             const int ago = S->ago + 1;
             int rb = 0;
             if (ago >= B.delay && ago % B.every == 0) rb = B.check ? moved : 1;
+            if (S->status & kErrTimeout) rb = 0;  // its bucket counts may be those of half a rebuild
             S->rebuild = rb;
             S->ago = rb ? 0 : ago;
             S->pending = defer;
@@ -265,8 +266,9 @@ void launch_integrate(cudaStream_t s, BoxDesc *boxes, const BatchUnits &u, const
 __global__ void k_force_rebuild_flag(BoxDesc *boxes, int nbox, int value)
 {
     for (int b = threadIdx.x; b < nbox; b += blockDim.x) {
-        boxes[b].st->rebuild = value;
-        if (value) boxes[b].st->ago = 0;
+        BoxState &S = *boxes[b].st;
+        S.rebuild = value && !(S.status & kErrTimeout);
+        if (value) S.ago = 0;
     }
 }
 

@@ -73,9 +73,16 @@ struct SmallPlan {
     const void *kernel = nullptr;
     int blocks = 0, rows = 0, parts = 0, lpr = 0, smem = 0;
 };
+// the launch's barrier waits: polls at most (a multiple of 1024, ~0.5 us each); barrier (tests): from
+// this one on, counted from 1 in each launch, one arrival more than there are blocks is waited for
+struct SmallWait {
+    unsigned polls = 1u << 22;  // ~2 s
+    unsigned barrier = 0;       // 0: none
+};
 bool small_run_plan(const BoxDesc &B, const StepConfig &c, SmallPlan &p);
 size_t small_bar_bytes();
-cudaError_t launch_small_run(cudaStream_t s, const BoxDesc &B, const SmallPlan &p, void *bar, int *done, long long nsteps);
+cudaError_t launch_small_run(cudaStream_t s, const BoxDesc &B, const SmallPlan &p, const SmallWait &w, void *bar,
+                             int *done, long long nsteps);
 // AoS x[3n] (and v[3n], or zero when null) -> components x[d], xh[d], v[d]; tags 1..n, type 1
 // and mask 1 into the arrays given (null: left as uploaded)
 void launch_load_state(cudaStream_t s, const double *xa, const double *va, int n, double *const x[3],
