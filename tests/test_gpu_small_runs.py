@@ -66,6 +66,23 @@ def test_boxes_that_share_a_run_kernel(style, large, small):
         bs[k].close()
 
 
+def test_a_smaller_box_leaves_an_earlier_box_its_one_launch_runs():
+    """the larger box's launch still goes through: with its barrier wait made to run out, its call says so
+    (on the step graph it would succeed)"""
+    for style, large, small in ((0, 3000, 2000), (0, 20000, 15000), (1, 20000, 15000)):
+        a, b = batch(large, style), batch(small, style)
+        for q in (a, b):
+            q.setup()
+            q.step(4)
+        assert mdpd.lib().mdpd_batch_test_run_wait(a.h, 8192, 3) == mdpd.OK
+        with pytest.raises(mdpd.MdpdError) as e:
+            a.step(4)
+        assert e.value.code == mdpd.ERR_TIMEOUT
+        b.step(4)
+        a.close()
+        b.close()
+
+
 # barriers of a step that rebuilds: 1 after integrate, 2 to 10 between and after the rebuild's passes (2: the
 # classes are counted, their counts not yet cleared), 11 after the density pass (mDPD), then the force pass's
 @pytest.mark.parametrize("style,barrier", [(0, k) for k in range(1, 13)] + [(1, k) for k in (1, 2, 5, 10, 11)])
