@@ -199,6 +199,10 @@ int mdpd_batch_set_shapes(mdpd_batch_t *b, int32_t shape_density, int32_t shape_
  * (from 1; 0: none) wait for an arrival that does not come.  Such a run ends with MDPD_ERR_TIMEOUT; its
  * box stays so: every later call that steps it or sets it up returns MDPD_ERR_TIMEOUT. */
 int mdpd_batch_test_run_wait(mdpd_batch_t *b, uint32_t polls, uint32_t barrier);
+/* for tests: of the batch's one-launch runs' launches (256 steps each at most), the launch-th from now on
+ * (from 1; 0: none) is answered as the device answers a launch that it has no room for; the steps from
+ * there on go by the step graph, with the same bits. */
+int mdpd_batch_test_refuse_run(mdpd_batch_t *b, int32_t launch);
 /* last per-step device time in milliseconds measured with CUDA events over nsteps */
 int mdpd_batch_time(mdpd_batch_t *b, int64_t nsteps, double *ms_per_step);
 /* nsteps un-captured steps with CUDA events around each kernel group (same kernels as the

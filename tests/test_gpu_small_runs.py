@@ -83,6 +83,25 @@ def test_a_smaller_box_leaves_an_earlier_box_its_one_launch_runs():
         b.close()
 
 
+@pytest.mark.parametrize("style", [0, 1])
+@pytest.mark.parametrize("launch", [1, 2, 3])
+def test_a_refused_launch_in_the_middle_of_a_run(style, launch):
+    """600 steps go in three launches; from the refused one on they go by the step graph: as many steps
+    and the same bits"""
+    a, b = batch(2500, style), batch(2500, style)
+    for q in (a, b):
+        q.setup()
+    assert mdpd.lib().mdpd_batch_test_refuse_run(a.h, launch) == mdpd.OK
+    for q in (a, b):
+        q.step(601)
+        assert q.thermo(0).step == 601
+        q.step(30)
+    assert same(a.state(0), b.state(0))
+    assert a.thermo(0).step == b.thermo(0).step == 631
+    a.close()
+    b.close()
+
+
 # barriers of a step that rebuilds: 1 after integrate, 2 to 10 between and after the rebuild's passes (2: the
 # classes are counted, their counts not yet cleared), 11 after the density pass (mDPD), then the force pass's
 @pytest.mark.parametrize("style,barrier", [(0, k) for k in range(1, 13)] + [(1, k) for k in (1, 2, 5, 10, 11)])

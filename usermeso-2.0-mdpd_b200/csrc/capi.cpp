@@ -732,6 +732,13 @@ int mdpd_batch_test_run_wait(mdpd_batch_t *b, uint32_t polls, uint32_t barrier)
     return MDPD_OK;
 }
 
+int mdpd_batch_test_refuse_run(mdpd_batch_t *b, int32_t launch)
+{
+    if (!b || launch < 0) return MDPD_ERR_ARG;
+    b->batch->refuse_run(launch);
+    return MDPD_OK;
+}
+
 int mdpd_jobs_validate(const char *spec_path, int32_t *njobs, uint64_t *bytes)
 {
     if (!spec_path) return MDPD_ERR_ARG;

@@ -777,7 +777,7 @@ void Batch::plan_small()
 // follow one another on the device: each waits for the end of the one launched before it (two could not
 // be resident together anyway), so no run can hold SMs that another one's unplaced blocks wait for.
 static cudaError_t ordered_small_run(cudaStream_t s, const BoxDesc &B, const SmallPlan &p, const SmallWait &w,
-                                     void *bar, int *done, long long nsteps)
+                                     void *bar, int *done, int nsteps)
 {
     static std::mutex mu;
     static cudaEvent_t last[64] = {};
@@ -797,19 +797,24 @@ void Batch::run(long long nsteps, bool sync, bool ev_last)
 {
     Range r("mdpd::run");
     const long long plain = nsteps - (ev_last && nsteps > 0 ? 1 : 0);
-    if (small_.kernel && plain > 0) {
-        const cudaError_t e = ordered_small_run(stream_, one_, small_, wait_, d_bar_, d_done, plain);
+    long long left = plain;
+    while (small_.kernel && left > 0) {
+        const int k = (int)std::min<long long>(left, kSmallRunSteps);
+        const bool refuse = refuse_ > 0 && --refuse_ == 0;
+        const cudaError_t e = refuse ? cudaErrorCooperativeLaunchTooLarge
+                                     : ordered_small_run(stream_, one_, small_, wait_, d_bar_, d_done, k);
         if (e != cudaSuccess) (void)cudaGetLastError();  // a refused launch is not left for the next caller
-        if (e == cudaErrorCooperativeLaunchTooLarge) {  // part of the device is taken (MPS): nothing was launched
-            small_.kernel = nullptr;
+        if (e == cudaErrorCooperativeLaunchTooLarge) {  // part of the device is taken (MPS): the steps not yet
+            small_.kernel = nullptr;                    // launched go by the step graph
             capture(0);
         } else {
             check_cuda(e, "run launch");
+            left -= k;
         }
     }
-    if (!small_.kernel) {
-        for (long long k = 0; k < plain; ++k) check_cuda(cudaGraphLaunch(graph_[0], stream_), "graph launch");
-        if (plain == nsteps && nsteps > 0 && defers()) {
+    if (left > 0) {
+        for (long long k = 0; k < left; ++k) check_cuda(cudaGraphLaunch(graph_[0], stream_), "graph launch");
+        if (plain == nsteps && defers()) {
             launch_finalize(stream_, d_boxes, units, 1);
             check_cuda(cudaGetLastError(), "finalize launch");
         }

@@ -158,6 +158,7 @@ public:
     // whether runs of plain steps go in one cooperative launch (k_small.cu) with the present shapes
     bool whole_runs() const { return small_.kernel != nullptr; }
     void set_run_wait(const SmallWait &w) { wait_ = w; }  // tests
+    void refuse_run(int launch) { refuse_ = launch; }        // tests
     const std::vector<Box *> &boxes() const { return boxes_; }
     StepConfig cfg;
     BatchUnits units;
@@ -170,6 +171,7 @@ private:
     BoxDesc one_;                  // a single box's descriptor as the passes see it
     SmallPlan small_;              // its whole-run launch (kernel: null when the box takes the graphs)
     SmallWait wait_;
+    int refuse_ = 0;               // tests: so many launches on, one is refused
     char *d_bar_ = nullptr;
     double *d_thermo = nullptr;
     BoxState *d_states = nullptr;  // gathered copies of the boxes' scalars

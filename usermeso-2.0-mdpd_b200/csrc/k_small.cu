@@ -28,7 +28,6 @@
 namespace mdpd {
 
 constexpr int kSmallWarps = 24, kSmallThreads = 32 * kSmallWarps;
-constexpr int kSmallMaxSteps = 256;           // steps per launch (their seeds are formed up front)
 
 struct SmallBar {
     unsigned arrived;
@@ -306,7 +305,7 @@ template <int STYLE, bool EXACT, bool UNI, int LPR>
 __global__ void __launch_bounds__(kSmallThreads, 1) k_run_box(const __grid_constant__ SmallArgs A)
 {
     extern __shared__ __align__(128) char s_dyn[];
-    __shared__ uint32_t s_seed[kSmallMaxSteps + 2];
+    __shared__ uint32_t s_seed[kSmallRunSteps + 2];
     __shared__ int s_w[kSmallWarps];
     __shared__ int s_flag[2];
     const BoxDesc &B = A.B;
@@ -518,10 +517,11 @@ bool small_run_plan(const BoxDesc &B, const StepConfig &c, SmallPlan &p)
 size_t small_bar_bytes() { return sizeof(SmallBar); }
 
 cudaError_t launch_small_run(cudaStream_t s, const BoxDesc &B, const SmallPlan &p, const SmallWait &w, void *bar,
-                             int *done, long long nsteps)
+                             int *done, int nsteps)
 {
     SmallArgs a;
     a.B = B;
+    a.nsteps = nsteps;
     a.bar = static_cast<SmallBar *>(bar);
     a.done = done;
     a.rows = p.rows;
@@ -529,16 +529,10 @@ cudaError_t launch_small_run(cudaStream_t s, const BoxDesc &B, const SmallPlan &
     a.nblocks = p.blocks;
     a.polls = w.polls;
     a.withhold = w.barrier ? w.barrier * (unsigned)p.blocks : 0xffffffffu;
-    while (nsteps > 0) {
-        a.nsteps = (int)std::min<long long>(nsteps, kSmallMaxSteps);
-        cudaError_t e = cudaMemsetAsync(bar, 0, sizeof(SmallBar), s);
-        if (e != cudaSuccess) return e;
-        void *args[] = {&a};
-        e = cudaLaunchCooperativeKernel(p.kernel, dim3(p.blocks), dim3(kSmallThreads), args, p.smem, s);
-        if (e != cudaSuccess) return e;
-        nsteps -= a.nsteps;
-    }
-    return cudaSuccess;
+    const cudaError_t e = cudaMemsetAsync(bar, 0, sizeof(SmallBar), s);
+    if (e != cudaSuccess) return e;
+    void *args[] = {&a};
+    return cudaLaunchCooperativeKernel(p.kernel, dim3(p.blocks), dim3(kSmallThreads), args, p.smem, s);
 }
 
 }  // namespace mdpd

@@ -67,8 +67,10 @@ void launch_density_half(cudaStream_t s, BoxDesc *boxes, const BatchUnits &u, co
 void launch_force_half(cudaStream_t s, BoxDesc *boxes, const BatchUnits &u, const StepConfig &c, int ev, int kick,
                        bool finish);
 // Whole runs of one small box in one cooperative launch (k_small.cu).  small_run_plan: whether the
-// box of a single-box batch is stepped so, and the launch's shape; launch_small_run: nsteps plain
-// steps (`bar`: small_bar_bytes() of device memory; done: the batch's counters)
+// box of a single-box batch is stepped so, and the launch's shape; launch_small_run: one launch of
+// nsteps plain steps, kSmallRunSteps at most (`bar`: small_bar_bytes() of device memory; done: the
+// batch's counters)
+constexpr int kSmallRunSteps = 256;  // their seeds are formed up front in shared memory
 struct SmallPlan {
     const void *kernel = nullptr;
     int blocks = 0, rows = 0, parts = 0, lpr = 0, smem = 0;
@@ -82,7 +84,7 @@ struct SmallWait {
 bool small_run_plan(const BoxDesc &B, const StepConfig &c, SmallPlan &p);
 size_t small_bar_bytes();
 cudaError_t launch_small_run(cudaStream_t s, const BoxDesc &B, const SmallPlan &p, const SmallWait &w, void *bar,
-                             int *done, long long nsteps);
+                             int *done, int nsteps);
 // AoS x[3n] (and v[3n], or zero when null) -> components x[d], xh[d], v[d]; tags 1..n, type 1
 // and mask 1 into the arrays given (null: left as uploaded)
 void launch_load_state(cudaStream_t s, const double *xa, const double *va, int n, double *const x[3],

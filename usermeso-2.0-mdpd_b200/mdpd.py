@@ -95,6 +95,7 @@ def lib():
             "mdpd_batch_tune_cached": ([vp, cp, i32p, i32p, i32p], C.c_int),
             "mdpd_batch_set_shapes": ([vp, i32, i32], C.c_int),
             "mdpd_batch_test_run_wait": ([vp, C.c_uint32, C.c_uint32], C.c_int),
+            "mdpd_batch_test_refuse_run": ([vp, i32], C.c_int),
             "mdpd_batch_time": ([vp, i64, dp], C.c_int),
             "mdpd_batch_profile": ([vp, i64, dp], C.c_int),
             "mdpd_batch_rebuild_steps": ([vp, C.POINTER(i64)], C.c_int),
