@@ -1,5 +1,6 @@
 """Runs of small boxes in one launch: several boxes, threads and refused launches side by side."""
 import threading
+import time
 
 import numpy as np
 import pytest
@@ -81,6 +82,79 @@ def test_a_smaller_box_leaves_an_earlier_box_its_one_launch_runs():
         b.step(4)
         a.close()
         b.close()
+
+
+def test_a_small_box_beside_a_large_one():
+    """calls of 1,000 steps of 2,000 particles from another thread do not keep a box of a million
+    particles from stepping, and the small box, stepped partly in one-launch runs and partly by the step
+    graph, keeps its bits"""
+    big, small, ref = batch(1000000), batch(2000, seed=5), batch(2000, seed=5)
+    for q in (big, small, ref):
+        q.setup()
+        q.step(300)
+
+    def fastest():
+        t = []
+        for _ in range(5):
+            a = time.perf_counter()
+            big.step(20)
+            t.append(time.perf_counter() - a)
+        return min(t)
+
+    alone = fastest()
+    stop, calls, errors = threading.Event(), [0], []
+
+    def go():
+        try:
+            while not stop.is_set():
+                small.step(1000)
+                calls[0] += 1
+        except Exception as e:  # seen by the main thread
+            errors.append(e)
+
+    th = threading.Thread(target=go)
+    th.start()
+    time.sleep(0.05)
+    beside = fastest()
+    time.sleep(0.1)  # the small box alone again
+    stop.set()
+    th.join()
+    assert not errors and calls[0] > 0
+    # one-launch runs beside it: about 20 times as long; step graphs: a few per cent
+    assert beside < 4 * alone
+    for _ in range(calls[0]):
+        ref.step(1000)
+    assert same(small.state(0), ref.state(0))
+    for q in (big, small, ref):
+        q.close()
+
+
+def test_small_boxes_of_several_threads_in_long_calls():
+    """calls long enough to change between one-launch runs and the step graph under way"""
+    sizes, steps = (2000, 3000, 2500), (1900, 700, 2600)
+
+    def go(k, out):
+        try:
+            b = batch(sizes[k], k % 2, seed=k + 1)
+            b.setup()
+            b.step(steps[k])
+            b.time(steps[k])  # plain steps only
+            out[k] = b.state(0) + (np.array([b.thermo(0).step]),)
+            b.close()
+        except Exception as e:  # seen by the main thread
+            out[k] = e
+
+    alone, together = {}, {}
+    for k in range(3):
+        go(k, alone)
+    th = [threading.Thread(target=go, args=(k, together)) for k in range(3)]
+    for t in th:
+        t.start()
+    for t in th:
+        t.join()
+    for k in range(3):
+        assert not isinstance(together[k], Exception), together[k]
+        assert same(alone[k], together[k]) and alone[k][2][0] == 2 * steps[k]
 
 
 @pytest.mark.parametrize("style", [0, 1])

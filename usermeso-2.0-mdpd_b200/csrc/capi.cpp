@@ -550,6 +550,7 @@ int mdpd_batch_time(mdpd_batch_t *b, int64_t nsteps, double *ms)
 {
     if (!b || !ms || nsteps <= 0) return MDPD_ERR_ARG;
     return guard(b->err, [&] {
+        const Stepping here;
         cudaEvent_t e0, e1;
         check_cuda(cudaEventCreate(&e0), "event");
         check_cuda(cudaEventCreate(&e1), "event");

@@ -7,6 +7,7 @@
 #include <mutex>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <numeric>
@@ -707,6 +708,7 @@ void Batch::capture(int ev)
 void Batch::setup()
 {
     Range r("mdpd::setup");
+    const Stepping here;
     launch_force_rebuild_flag(stream_, d_boxes, units.nbox, 1);
     launch_rebuild(stream_, d_boxes, units, cfg, d_done);
     if (cfg.style == 0) launch_density(stream_, d_boxes, units, cfg);
@@ -731,6 +733,7 @@ void Batch::setup_boxes(const std::vector<int> &which)
 {
     Range r("mdpd::setup");
     if (which.empty()) return;
+    const Stepping here;
     int *d = batch_alloc<int>(which.size(), stream_);
     check_cuda(cudaMemcpyAsync(d, which.data(), sizeof(int) * which.size(), cudaMemcpyHostToDevice, stream_),
                "setup boxes");
@@ -773,18 +776,36 @@ void Batch::plan_small()
     if (small_.kernel && !d_bar_) d_bar_ = batch_alloc<char>(small_bar_bytes(), stream_);
 }
 
-// A small box's run needs a block on every SM at once.  Runs of several streams and threads therefore
-// follow one another on the device: each waits for the end of the one launched before it (two could not
-// be resident together anyway), so no run can hold SMs that another one's unplaced blocks wait for.
+constexpr int kMaxDevices = 64;
+static std::atomic<int> g_stepping[kMaxDevices];
+static thread_local int t_stepping[kMaxDevices];
+
+Stepping::Stepping()
+{
+    check_cuda(cudaGetDevice(&dev_), "device");
+    if (dev_ < 0 || dev_ >= kMaxDevices) throw std::runtime_error("CUDA device ordinal out of range");
+    if (t_stepping[dev_]++ == 0) ++g_stepping[dev_];
+}
+
+Stepping::~Stepping()
+{
+    if (--t_stepping[dev_] == 0) --g_stepping[dev_];
+}
+
+bool Stepping::alone() const { return g_stepping[dev_].load() == 1; }
+
+// A small box's run needs a block on every SM at once.  Should two be queued from different streams, each
+// waits for the end of the one launched before it (two could not be resident together anyway), so no run
+// can hold SMs that another one's unplaced blocks wait for.
 static cudaError_t ordered_small_run(cudaStream_t s, const BoxDesc &B, const SmallPlan &p, const SmallWait &w,
                                      void *bar, int *done, int nsteps)
 {
     static std::mutex mu;
-    static cudaEvent_t last[64] = {};
+    static cudaEvent_t last[kMaxDevices] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+    if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
     std::lock_guard<std::mutex> lock(mu);
     if (!last[dev] && (e = cudaEventCreateWithFlags(&last[dev], cudaEventDisableTiming)) != cudaSuccess) return e;
     if ((e = cudaStreamWaitEvent(s, last[dev], 0)) != cudaSuccess) return e;
@@ -797,27 +818,46 @@ void Batch::run(long long nsteps, bool sync, bool ev_last)
 {
     Range r("mdpd::run");
     const long long plain = nsteps - (ev_last && nsteps > 0 ? 1 : 0);
+    // A one-launch run holds every SM for up to kSmallRunSteps steps, so a small box takes them only while
+    // no other thread steps boxes on the device: its step graph leaves most of the chip to the others.
+    // Measured (steps/s): 2M particles beside a 2,000-particle box 838 on graphs, 39 beside one-launch runs
+    // (alone 851); four threads with 20,000 particles each 40,000 and 28,000 together, with 2,000 each 57,000
+    // and 43,000; two threads with 2,000 each 39,400 and 42,700, with 3,000 DPD particles each 37,500 and
+    // 53,200 (a launch per pass and no overlap would be 22,000 and 20,000).  Whether that holds is asked again
+    // every kSmallRunSteps steps, with one launch at most under way: a call of 20 steps beside one of 60,000
+    // waits 5 ms, not for the end of the other.
+    const Stepping here;
     long long left = plain;
-    while (small_.kernel && left > 0) {
+    bool deferred = false;  // graph steps whose last half-kick is still to be applied
+    while (left > 0) {
         const int k = (int)std::min<long long>(left, kSmallRunSteps);
+        if (!small_.kernel || !here.alone()) {
+            if (!graph_[0]) capture(0);
+            for (int q = 0; q < k; ++q) check_cuda(cudaGraphLaunch(graph_[0], stream_), "graph launch");
+            deferred = defers();
+            left -= k;
+            continue;
+        }
+        if (deferred) {
+            launch_finalize(stream_, d_boxes, units, 1);
+            check_cuda(cudaGetLastError(), "finalize launch");
+            deferred = false;
+        }
         const bool refuse = refuse_ > 0 && --refuse_ == 0;
         const cudaError_t e = refuse ? cudaErrorCooperativeLaunchTooLarge
                                      : ordered_small_run(stream_, one_, small_, wait_, d_bar_, d_done, k);
         if (e != cudaSuccess) (void)cudaGetLastError();  // a refused launch is not left for the next caller
         if (e == cudaErrorCooperativeLaunchTooLarge) {  // part of the device is taken (MPS): the steps not yet
             small_.kernel = nullptr;                    // launched go by the step graph
-            capture(0);
-        } else {
-            check_cuda(e, "run launch");
-            left -= k;
+            continue;
         }
+        check_cuda(e, "run launch");
+        left -= k;
+        if (left > 0) check_cuda(cudaStreamSynchronize(stream_), "run");
     }
-    if (left > 0) {
-        for (long long k = 0; k < left; ++k) check_cuda(cudaGraphLaunch(graph_[0], stream_), "graph launch");
-        if (plain == nsteps && defers()) {
-            launch_finalize(stream_, d_boxes, units, 1);
-            check_cuda(cudaGetLastError(), "finalize launch");
-        }
+    if (deferred && plain == nsteps) {
+        launch_finalize(stream_, d_boxes, units, 1);
+        check_cuda(cudaGetLastError(), "finalize launch");
     }
     if (plain < nsteps) check_cuda(cudaGraphLaunch(graph_[1], stream_), "graph launch");
     if (sync) check_cuda(cudaStreamSynchronize(stream_), "run");
@@ -835,6 +875,7 @@ long long Batch::rebuild_steps()
 double Batch::time_pair_passes(int reps)
 {
     Range r("mdpd::time_pair_passes");
+    const Stepping here;
     cudaEvent_t e0, e1;
     check_cuda(cudaEventCreate(&e0), "event");
     check_cuda(cudaEventCreate(&e1), "event");
@@ -857,6 +898,7 @@ double Batch::time_pair_passes(int reps)
 
 void Batch::profile(long long nsteps, double out[5])
 {
+    const Stepping here;
     cudaEvent_t ev[5];
     for (auto &e : ev) check_cuda(cudaEventCreate(&e), "event");
     double acc[4] = {0, 0, 0, 0};
@@ -946,6 +988,7 @@ void Batch::to_thermo(const double *h, const BoxState *sts, std::vector<Thermo> 
 void Batch::run_thermo(long long nsteps, const std::function<void(long long, const std::vector<Thermo> &)> &sink)
 {
     Range r("mdpd::run_thermo");
+    const Stepping here;
     const int nb = (int)boxes_.size();
     const size_t part_bytes = sizeof(double) * kPartialStride * nb, st_bytes = sizeof(BoxState) * nb;
     if (!h_stage_) {

@@ -199,6 +199,20 @@ struct Range {
     Range &operator=(const Range &) = delete;
 };
 
+// Counts the threads of this process whose call steps or sets up boxes on the current device, from its
+// first launch to its wait (scopes of one thread nest and count once).
+class Stepping {
+public:
+    Stepping();
+    ~Stepping();
+    Stepping(const Stepping &) = delete;
+    Stepping &operator=(const Stepping &) = delete;
+    bool alone() const;  // no other thread's call is under way
+
+private:
+    int dev_ = 0;
+};
+
 std::string status_text(int bits);  // names of the set bits of a box status word
 std::string cuda_err(cudaError_t e);
 void check_cuda(cudaError_t e, const char *what);

@@ -1101,6 +1101,7 @@ void Script::read_data(const std::string &path)
 void Script::run(long long nsteps)
 {
     ensure_device();
+    const Stepping here;
     // setup (ModifiedVerlet::setup): rebuild, density, forces with energy/virial
     batch_->setup();
     step_ = box_->state().step;

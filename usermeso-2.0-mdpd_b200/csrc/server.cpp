@@ -347,9 +347,12 @@ void mdpd_server_s::loop()
         Range chunk_range("mdpd::server_chunk");
         const double tk0 = now();
         cudaEventRecord(e0, batch->stream());
-        batch->run(k, false, true);  // a retiring job's thermo reports its last step's energy and virial
-        cudaEventRecord(e1, batch->stream());
-        cudaEventSynchronize(e1);
+        {
+            const Stepping here;
+            batch->run(k, false, true);  // a retiring job's thermo reports its last step's energy and virial
+            cudaEventRecord(e1, batch->stream());
+            cudaEventSynchronize(e1);
+        }
         float ms = 0;
         cudaEventElapsedTime(&ms, e0, e1);
         long long nparts = 0;
