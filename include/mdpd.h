@@ -183,7 +183,7 @@ int mdpd_batch_tune(mdpd_batch_t *b, int32_t *shape_density, int32_t *shape_forc
  * passes, ms per evaluation).  The key
  * names the workload class the pick applies to: GPU model and SM count, pass family and options,
  * mean density (0.25 steps), neighbour cutoff (0.05 steps), total particles and box count (powers
- * of two).  A stored key is applied without timing (*cached = 1); otherwise the batch is timed
+ * of two); full-list boxes whose runs go in one launch have keys of their own.  A stored key is applied without timing (*cached = 1); otherwise the batch is timed
  * as by mdpd_batch_tune and its pick added to the file (*cached = 0), which is rewritten
  * whole through a temporary and a rename, keeping the other members.  A malformed file or entry
  * returns MDPD_ERR_PARSE and is left untouched.  The reference's ThreadTuner learns online and

@@ -1,4 +1,5 @@
 """Runs of small boxes in one launch: several boxes, threads and refused launches side by side."""
+import json
 import threading
 import time
 
@@ -215,3 +216,29 @@ def test_a_barrier_wait_that_runs_out(style, barrier):
     assert same(other.state(0), ref.state(0))
     other.close()
     ref.close()
+
+
+def test_tune_cache_keeps_boxes_with_one_launch_runs_apart(tmp_path):
+    """140,000 and 250,000 DPD particles lie in one power of two; the first box's runs go in one launch at
+    one thread per particle, the second's do not: neither takes the other's stored pick"""
+    cache = tmp_path / "tune.json"
+    sizes = (140000, 250000)  # one-launch runs: up to 1,400 rows on each of 148 SMs
+    for order in (sizes, sizes[::-1]):
+        if cache.exists():
+            cache.unlink()
+        for n in order:
+            b = batch(n, 1)
+            b.setup()
+            d, f, hit = b.tune(cache=cache)
+            assert not hit and (n == sizes[1] or (d, f) == (1, 1))
+            b.close()
+            # what is stored now is another shape than the next box would take by the rule
+            j = json.loads(cache.read_text())
+            for e in j["entries"].values():
+                e["density"], e["force"] = 2, 4
+            cache.write_text(json.dumps(j))
+        assert len(j["entries"]) == 2
+    b = batch(sizes[1], 1)  # an entry of its own class is applied
+    b.setup()
+    assert b.tune(cache=cache) == (2, 4, True)
+    b.close()

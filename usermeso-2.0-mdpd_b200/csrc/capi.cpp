@@ -630,7 +630,8 @@ static TunePick tune_by_timing(mdpd_batch_s *b)
 
 // the workload class a stored pick applies to: GPU model and SM count, the pass family and
 // its options, mean density (0.25 steps), neighbour cutoff (0.05 steps), total particles and
-// box count (powers of two)
+// box count (powers of two); a full-list box whose runs go in one launch at one thread per particle, which
+// ends within a power of two, has a class of its own (its pick is not timed against other shapes)
 static std::string tune_key(mdpd_batch_s *b)
 {
     const Batch &bt = *b->batch;
@@ -650,6 +651,7 @@ static std::string tune_key(mdpd_batch_s *b)
     if (c.aboundary) fam += " +aboundary";
     if (c.exact_rng) fam += " +exact-rng";
     if (!c.uniform_types) fam += " +types";
+    if (!c.half && bt.whole_runs_at_one()) fam += " +one-launch runs";
     const int nb = (int)bt.boxes().size();
     char buf[512];
     std::snprintf(buf, sizeof buf, "%s sm%d | %s | rho %.2f | rc %.2f | particles 2^%d | boxes 2^%d", prop.name,

@@ -776,6 +776,14 @@ void Batch::plan_small()
     if (small_.kernel && !d_bar_) d_bar_ = batch_alloc<char>(small_bar_bytes(), stream_);
 }
 
+bool Batch::whole_runs_at_one() const
+{
+    StepConfig c = cfg;
+    c.tpp_density = c.tpp_force = 1;
+    SmallPlan p;
+    return boxes_.size() == 1 && small_run_plan(one_, c, p);
+}
+
 constexpr int kMaxDevices = 64;
 static std::atomic<int> g_stepping[kMaxDevices];
 static thread_local int t_stepping[kMaxDevices];

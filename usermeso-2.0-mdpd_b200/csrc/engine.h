@@ -157,6 +157,8 @@ public:
     cudaStream_t stream() const { return stream_; }
     // whether runs of plain steps go in one cooperative launch (k_small.cu) with the present shapes
     bool whole_runs() const { return small_.kernel != nullptr; }
+    // the same with one thread per particle in the full-list passes
+    bool whole_runs_at_one() const;
     void set_run_wait(const SmallWait &w) { wait_ = w; }  // tests
     void refuse_run(int launch) { refuse_ = launch; }        // tests
     const std::vector<Box *> &boxes() const { return boxes_; }
