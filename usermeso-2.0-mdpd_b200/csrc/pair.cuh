@@ -46,7 +46,9 @@ __device__ __forceinline__ float pair_scalar(const PairCoeff &cf, float dx, floa
         fpair = (cf.A * wc + cf.B * (rho_i + rho_j) * wcr) - gam * wc * wc * dot * rinv + sig * wc * rn * dtis;
         if (EV) ev.pe += cf.e_cut * wc * wc + cf.e_cut_r * (rho_i + rho_j) * wcr * wcr;
     } else {
-        const float wr = cf.expw == 1.f ? wc : __powf(wc, cf.expw);
+        // just inside a cutoff other than 1, r * inv_cut can round above 1: no weight there, not the power
+        // of a negative number
+        const float wr = cf.expw == 1.f ? wc : wc > 0.f ? __powf(wc, cf.expw) : 0.f;
         fpair = cf.A * wc - gam * wr * wr * dot * rinv + sig * wr * rn * dtis;
         if (EV) ev.pe += cf.e_cut * wc * wc;
     }
