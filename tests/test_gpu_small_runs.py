@@ -242,3 +242,37 @@ def test_tune_cache_keeps_boxes_with_one_launch_runs_apart(tmp_path):
     b.setup()
     assert b.tune(cache=cache) == (2, 4, True)
     b.close()
+
+
+def edge(kind):
+    """specs of the last box whose runs go in one launch on 148 SMs, and of the first that does not"""
+    if kind == "rows mdpd":  # 768 rows per block: each warp of the force pass holds 32
+        return [mdpd.box_spec(n, (n / 6.05) ** (1 / 3), seed=2, init_seed=8) for n in (148 * 768, 148 * 768 + 1)]
+    if kind == "rows dpd":  # 1,400 rows per block: shared memory is nearly full
+        return [mdpd.box_spec(n, (n / 3.0) ** (1 / 3), seed=2, init_seed=8, **DPD) for n in (148 * 1400, 148 * 1400 + 1)]
+    # 22^3 bins, mostly empty: as many as particles and 4,096 more
+    return [mdpd.box_spec(n, 26.0, seed=2, init_seed=8, fill_lo=(12.2, 0, 0), fill_hi=(13.8, 26, 26))
+            for n in (22 ** 3 - 4096, 22 ** 3 - 4097)]
+
+
+@pytest.mark.parametrize("kind", ["rows mdpd", "rows dpd", "bins"])
+def test_the_last_box_with_one_launch_runs_and_the_first_without(kind):
+    """plain steps and steps with a thermo line each (always launches of their passes): the same bits"""
+    for spec, one_launch in zip(edge(kind), (True, False)):
+        a, b = mdpd.Batch([spec]), mdpd.Batch([spec])
+        for q in (a, b):
+            q.setup()
+        a.step(14)
+        b.run_thermo(14)
+        assert same(a.state(0), b.state(0))
+        assert a.thermo(0).nbuild == b.thermo(0).nbuild >= 3 and a.thermo(0).status == 0
+        # which way the plain steps went: only one-launch runs meet a barrier
+        mdpd.lib().mdpd_batch_test_run_wait(a.h, 8192, 1)
+        if one_launch:
+            with pytest.raises(mdpd.MdpdError) as e:
+                a.step(2)
+            assert e.value.code == mdpd.ERR_TIMEOUT
+        else:
+            a.step(2)
+        a.close()
+        b.close()
