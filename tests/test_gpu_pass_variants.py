@@ -135,22 +135,6 @@ def test_steps_of_one_run_same_bits_as_single_runs(exact):
     b.close()
 
 
-def wall_box(n_side, exact):
-    """fluid between frozen walls at the low and high x ends"""
-    L = np.array([n_side, 5.0, 5.0])
-    rng = np.random.default_rng(4)
-    nf, nw = int(6.05 * (L[0] - 4) * 25), int(8 * 4 * 25)
-    xf = rng.uniform(0, 1, (nf, 3)) * (L - (4, 0, 0)) + (2, 0, 0)
-    xw = rng.uniform(0, 1, (nw, 3)) * (4, 5, 5)
-    xw[:, 0] = np.mod(xw[:, 0] - 2, L[0])
-    v = np.concatenate([rng.normal(0, 1, (nf, 3)), np.zeros((nw, 3))])
-    return deck((nf, nw), (0,) * 3, L, "group fluid type 1\ngroup solid type 2",
-                "pair_style mdpd/meso 1.0 1.0 77 fluid solid\npair_coeff * * -20 15 4.5 1.0 0.75\n"
-                f"pair_modify rng {exact}",
-                "fix BC all aboundary/rho/meso cut_rho 0.75 phi_c 0.5 cut_phi 1.0 rho_wall 8.0 wall solid mobile fluid\n"
-                "fix NVE fluid nve/meso", np.concatenate([xf, xw]), v)
-
-
 def dpd_box(n, exact):
     L = (n / 3.0) ** (1 / 3)
     x, v = lattice(n, L, 6)
@@ -170,7 +154,7 @@ def mdpd_box(n, exact):
 
 
 # one block per SM holds 1/148 of the rows: boxes at the edges of the lanes-per-row ranges (24 and 96
-# rows per block on a B200), below and above one row per block, and past the run kernel's range
+# rows per block on a B200), below and above one row per block, and some way into the range of two lanes
 @pytest.mark.parametrize("exact", ["fast", "exact"])
 @pytest.mark.parametrize("n", [401, 3552, 3553, 14208, 14209, 30011, 70001])
 @pytest.mark.parametrize("make", [mdpd_box, dpd_box])

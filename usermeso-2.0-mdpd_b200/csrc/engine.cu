@@ -85,6 +85,8 @@ size_t Box::estimate_bytes(const Spec &spec, int n)
     const long long nbin = (long long)g.mbin[0] * g.mbin[1] * g.mbin[2];
     const long long gc = ghost_estimate(spec, g, n);
     const long long nrow = ceil_to(n, 32);
+    // An upper bound, kept as jobs have been admitted and placed by it: the arena holds the force once, no
+    // bins of ghosts and two scan buffers of a few words, which is less.
     size_t b = 0;
     b += (size_t)n * (2 * 6 * 8 + 3 * 8 + 2 * 16 + 6 * 4 + 2 * 4 + 3 * 4 + 4);  // x,v,xh,f,tag/type/mask,phi,cls,sub,perm,count
     b += (size_t)(n + gc) * (16 + 16 + 4 + 4 + 4 + 16 + 4);                      // pos, vel, rho, bin_of, bin_order, bpos, gfirst
